@@ -440,11 +440,12 @@ def run_reference(args):
         return 0
     sys.path.insert(0, os.path.join(ROOT, "oracle"))
     import ref_runner
-    if not ref_runner.reference_available():
-        print(json.dumps({"impl": "reference", "unavailable": "reference build oracle/_ref missing"}))
-        return 0
+    # a workload the reference cannot render says so whether its build is here or not
     if WORKLOAD.get("no_reference"):
         print(json.dumps({"impl": "reference", "unavailable": WORKLOAD["no_reference"]}))
+        return 0
+    if not ref_runner.reference_available():
+        print(json.dumps({"impl": "reference", "unavailable": "reference build oracle/_ref missing"}))
         return 0
     small = build_workload(REF_RES, spp=1)
     for i in range(args.warmup):  # warm-up on a 32x32 slice: pages in, starts the pool
