@@ -207,10 +207,13 @@ def kernel_bytes(kernel, wl, work):
     if kernel == "k_edge_tasks":
         return (work["tasks"] * (24 + POINT_BYTES) + (I - work["items_first_stage"]) * 20 +
                 work["visits_tasks"] * NODE_BYTES)
-    # the level walk of the same subtrees: the points' contexts, the subtrees'
-    # nodes, the items of their leaves
+    # the warp walk: the points' contexts, their trees' nodes and the items of
+    # their leaves
     if kernel == "k_walk_ctx":
         return P * POINT_BYTES
+    if kernel == "k_edge_walk":
+        return work["visits_tasks"] * NODE_BYTES + I * 20
+    # the walk level by level (profiles of earlier builds)
     if kernel == "k_edge_level":
         return work["tasks"] * 24 + work["visits_tasks"] * NODE_BYTES
     if kernel == "k_edge_leaves":

@@ -97,7 +97,7 @@ struct EdgeStats {
 
 struct BackwardQueues {
     DevBuf pt, items, item_w, item_dp, pt_last, pt_items, counts, survivors, hits, side_rad, tasks, tasks2;
-    DevBuf walk_ctx, leafq;  // the level walk of the subtrees
+    DevBuf walk_ctx, packets;  // the warp walk: the points' contexts, its rounds' packets
     DevBuf line_ctx;         // the points' line-sample setups
     long long cap_items = 0;     // grown on overflow, kept with the buffers
     double points_per_sample = 1;  // shading points per pixel sample the last overflow asked for
@@ -211,7 +211,7 @@ struct dr_scene {
     // lists and scratch, and the arena of the results
     bool gpu_edges = false;
     DevBuf edge_topo, edge_lists, edge_scratch, edge_arena;
-    DevBuf edge_recs;  // silhouette-test records of both trees' edges
+    DevBuf edge_recs;  // silhouette-test records of both trees' edges; the children of large trees' nodes
     size_t num_sil_edges = 0, num_nrm_edges = 0;
     int topo_count = 0;
     bool topo_dev_valid = false;
@@ -283,6 +283,14 @@ void upload_arena(DevBuf &arena, const ArenaLayout &lay, cudaStream_t st) {
 
 void build_edges_gpu(dr_scene *sc, cudaStream_t st);
 void build_edge_records(dr_scene *sc, cudaStream_t st);
+
+// Edge trees above this many nodes are walked by warps (k_edge_walk) or, with
+// the depth-first tuning, in two stages (k_edge_expand, k_edge_tasks): their
+// points' walks are long and uneven.
+constexpr int kSplitTraversalNodes = 4096;
+bool split_trees(const DevScene &ds) {
+    return ds.num_sil_nodes > kSplitTraversalNodes || ds.num_nrm_nodes > kSplitTraversalNodes;
+}
 
 void upload_scene(dr_scene *sc, cudaStream_t st, bool refit = false) {
     HostScene &h = sc->h;
@@ -385,17 +393,32 @@ void upload_scene(dr_scene *sc, cudaStream_t st, bool refit = false) {
     build_edge_records(sc, st);
 }
 
-// The silhouette-test records of both trees' edges (after every build).
+// The silhouette-test records of both trees' edges and, for trees walked by
+// warps, the interior nodes' children side by side (after every build).
 void build_edge_records(dr_scene *sc, cudaStream_t st) {
     const size_t ns = sc->num_sil_edges, nn = sc->num_nrm_edges;
-    sc->edge_recs.reserve(sizeof(EdgeRec) * std::max<size_t>(1, ns + nn));
+    const size_t rec_bytes = (sizeof(EdgeRec) * std::max<size_t>(1, ns + nn) + 255) & ~size_t(255);
+    const bool split = split_trees(sc->ds);
+    const size_t s4 = split ? 4 * (size_t)sc->ds.num_sil_nodes : 0, n4 = split ? 4 * (size_t)sc->ds.num_nrm_nodes : 0;
+    sc->edge_recs.reserve(rec_bytes + sizeof(float4) * (s4 + 2 * n4));
     EdgeRec *r = sc->edge_recs.as<EdgeRec>();
     check_cuda(dr_launch_edge_records(sc->ds, sc->ds.sil_edges, (int)ns, r, st), "edge records");
     check_cuda(dr_launch_edge_records(sc->ds, sc->ds.nrm_edges, (int)nn, r + ns, st), "edge records");
-    check_cuda(cudaStreamSynchronize(st), "edge records");
     sc->last_launches += 2;
     sc->ds.sil_rec = r;
     sc->ds.nrm_rec = r + ns;
+    sc->ds.sil_box = sc->ds.nrm_box = sc->ds.nrm_dir = nullptr;
+    if (split) {
+        float4 *k = reinterpret_cast<float4 *>((char *)sc->edge_recs.p + rec_bytes);
+        check_cuda(dr_launch_edge_children(sc->ds.sil_nodes, sc->ds.num_sil_nodes, k, nullptr, st), "edge children");
+        check_cuda(dr_launch_edge_children(sc->ds.nrm_nodes, sc->ds.num_nrm_nodes, k + s4, k + s4 + n4, st),
+                   "edge children");
+        sc->last_launches += 2;
+        sc->ds.sil_box = k;
+        sc->ds.nrm_box = k + s4;
+        sc->ds.nrm_dir = k + s4 + n4;
+    }
+    check_cuda(cudaStreamSynchronize(st), "edge records");
 }
 
 // Edges of a flattened tree: the last node in depth-first order is a leaf
@@ -529,12 +552,13 @@ void collect_timings(dr_scene *sc, cudaStream_t st) {
     }
 }
 
-// Edge trees above this many nodes are walked in two stages (k_edge_expand,
-// k_edge_tasks): their points' walks are long and uneven.
-constexpr int kSplitTraversalNodes = 4096;
-// Queues of the two-stage walk (the first stage's subtrees, each level's nodes
-// in two halves by class, the leaves): up to 128 entries per point, at most
-// 4 GiB each; a node that finds no room is walked depth first by its lane.
+// Packets each round of the warp walk can hand on (32 pending nodes each): 4
+// per point, between 16 K (9 MB a queue) and 1 M (570 MB a queue); a warp that
+// finds no room walks on itself.
+constexpr long long kMinPackets = 1 << 14, kMaxPackets = 1 << 20;
+// Queues of the depth-first walk (the first stage's subtrees, and those handed
+// on between rounds): up to 128 entries per point, at most 4 GiB each; a
+// subtree that finds no room is walked by its lane.
 constexpr long long kTasksPerPoint = 128, kMaxTasks = (4ll << 30) / sizeof(EdgeTask);
 
 // The scene's device view with this call's per-render settings.
@@ -544,7 +568,7 @@ DevScene call_scene(const dr_scene *sc, const dr_render_desc *rd) {
     ds.detached_pdf = (rd->flags & DR_FLAG_DETACHED_PDF) != 0;
     ds.edge_lobe_mis = (rd->flags & DR_FLAG_EDGE_LOBE_MIS) != 0;
     ds.specular_chains = sc->h.specular_bounces && rd->max_bounces >= 1;
-    ds.split_traversal = sc->ds.num_sil_nodes > kSplitTraversalNodes || sc->ds.num_nrm_nodes > kSplitTraversalNodes;
+    ds.split_traversal = split_trees(sc->ds);
     return ds;
 }
 
@@ -923,7 +947,6 @@ std::pair<long long, long long> run_backward(dr_scene *scene, const dr_render_de
     work[1] = items;
     work[6] = (long long)c.visits_walk;
     work[7] = (long long)c.visits_tasks;
-    work[9] = (long long)c.spilled;
     std::memcpy(scene->last_work, work, sizeof(work));
     return {P, items};
 }
@@ -1095,7 +1118,7 @@ void backward_on_queues(dr_scene *scene, const dr_render_desc *rd, const DevScen
     BackwardWorkspace ws{};
     ws.hand_steps = scene->tune.hand_steps;
     ws.task_rounds = scene->tune.task_rounds;
-    ws.level_walk = scene->tune.depth_first ? 0 : 1;
+    const bool depth_first = scene->tune.depth_first != 0;
     const bool split = view ? view->split_traversal : call_scene(scene, rd).split_traversal;
     const bool lbvh = (view ? view->num_tris : call_scene(scene, rd).num_tris) > DR_LINEAR_TRIS;
     auto bind_items = [&]() {
@@ -1121,9 +1144,12 @@ void backward_on_queues(dr_scene *scene, const dr_render_desc *rd, const DevScen
         ws.pt_last = q.pt_last.as<unsigned long long>();
         q.pt_items.reserve(sizeof(int) * cap_points);
         ws.pt_items = q.pt_items.as<int>();
-        if (split && ws.level_walk) {
+        if (split && !depth_first) {
             q.walk_ctx.reserve(sizeof(float4) * DR_CTX_F4 * cap_points);
             ws.walk_ctx = q.walk_ctx.as<float4>();
+            ws.cap_packets = std::min(kMaxPackets, std::max(kMinPackets, 4 * cap_points));
+            q.packets.reserve((size_t)DR_WALK_PACKET_BYTES * 2 * ws.cap_packets);
+            ws.packets = q.packets.p;
         }
         if (lbvh) {
             q.line_ctx.reserve(sizeof(float4) * DR_LCTX_F4 * cap_points);
@@ -1134,18 +1160,13 @@ void backward_on_queues(dr_scene *scene, const dr_render_desc *rd, const DevScen
     bind_points();
     ws.counters = q.counts.as<BackwardCounters>();
     bind_items();
-    if (split) {
+    if (split && depth_first) {
         long long cap_tasks = std::min(kMaxTasks, std::max(1ll << 16, kTasksPerPoint * cap_points));
         q.tasks.reserve(sizeof(EdgeTask) * cap_tasks);
         q.tasks2.reserve(sizeof(EdgeTask) * cap_tasks);
         ws.tasks = q.tasks.as<EdgeTask>();
         ws.tasks2 = q.tasks2.as<EdgeTask>();
         ws.cap_tasks = cap_tasks;
-        if (ws.level_walk) {
-            q.leafq.reserve(sizeof(EdgeTask) * cap_tasks);
-            ws.leafq = q.leafq.as<EdgeTask>();
-            ws.cap_leaves = cap_tasks;
-        }
     }
     // the item queue grows to what the traversal reported, up to its limit
     // (the grown queue is kept for later calls)

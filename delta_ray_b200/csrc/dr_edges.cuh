@@ -96,10 +96,10 @@ DEV int cone_poly(int lookup, int i) {
     return (int)((w >> (4 * (n - 1 - i))) & 0xF);
 }
 
-DEV_NOINLINE bool box_cone(const float *lo, const float *hi, const ConeSpec &cone) {
+DEV bool box_cone_box(float3 lo, float3 hi, const ConeSpec &cone) {
     if (cone.cos_angle <= 0.f) return true;
-    float3 C = f3(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]));
-    float3 E = f3(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]));
+    float3 C = f3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
+    float3 E = f3(0.5f * (hi.x - lo.x), 0.5f * (hi.y - lo.y), 0.5f * (hi.z - lo.z));
     float3 CmV = C - cone.o;
     float DdCmV = dot(cone.d, CmV);
     float rad = E.x * fabsf(cone.d.x) + E.y * fabsf(cone.d.y) + E.z * fabsf(cone.d.z);
@@ -169,6 +169,9 @@ DEV_NOINLINE bool box_cone(const float *lo, const float *hi, const ConeSpec &con
     }
     return false;
 }
+DEV_NOINLINE bool box_cone(const float *lo, const float *hi, const ConeSpec &cone) {
+    return box_cone_box(f3(lo[0], lo[1], lo[2]), f3(hi[0], hi[1], hi[2]), cone);
+}
 
 // ---------------------------------------------------------------------------
 // Edge-tree node bounds
@@ -231,22 +234,21 @@ DEV float filt_log2(float x) { return log2f(x); }
 DEV float filt_exp2(float x) { return exp2f(x); }
 #endif
 
-// The corners' products with a direction, per axis: corner i has the hi
-// coordinate on axis a iff bit a of i is set, and dot(d, corner_i - p) is
-// (x[i & 1] + y[(i >> 1) & 1]) + z[i >> 2], the bits of the per-corner dot.
-struct CornerDots {
-    float x[2], y[2], z[2];
-    DEV float at(int i) const { return (x[i & 1] + y[(i >> 1) & 1]) + z[i >> 2]; }
+// The largest and the smallest of dot(d, corner - p) over a box's corners,
+// q: lo - p, hi - p per axis (x0 x1 y0 y1 z0 z1).  Each corner's dot is
+// (x + y) + z with one product per axis, and a rounded sum does not fall when
+// a term grows, so the extreme corner takes the extreme product of each axis:
+// two sums instead of eight per extreme, with the bits of the corner loop
+// (a zero's sign aside, which no use of them tells apart).
+struct DotRange {
+    float lo, hi;
 };
-DEV CornerDots corner_dots(float3 d, const float *q) {  // q: lo - p, hi - p per axis (x0 x1 y0 y1 z0 z1)
-    CornerDots c;
-    c.x[0] = d.x * q[0];
-    c.x[1] = d.x * q[1];
-    c.y[0] = d.y * q[2];
-    c.y[1] = d.y * q[3];
-    c.z[0] = d.z * q[4];
-    c.z[1] = d.z * q[5];
-    return c;
+DEV DotRange corner_range(float3 d, const float *q) {
+    const float x0 = d.x * q[0], x1 = d.x * q[1], y0 = d.y * q[2], y1 = d.y * q[3], z0 = d.z * q[4], z1 = d.z * q[5];
+    DotRange r;
+    r.lo = (fminf(x0, x1) + fminf(y0, y1)) + fminf(z0, z1);
+    r.hi = (fmaxf(x0, x1) + fmaxf(y0, y1)) + fmaxf(z0, z1);
+    return r;
 }
 
 // fast_m (may be null) asks for the filtered form, used where only the
@@ -258,28 +260,17 @@ DEV CornerDots corner_dots(float3 d, const float *q) {  // q: lo - p, hi - p per
 // evaluated on the same hdn and *fast_m is 0; otherwise the returned bound is
 // on the exact one's side of 1 and of 0, within relative m of it, and *fast_m
 // is m.  Without fast_m, or for other lobes, the exact bound (*fast_m 0).
-DEV_NOINLINE float bsdf_bound(const DevEdgeNode &node, const BoundCtx &c, float *fast_m = nullptr) {
+DEV float bsdf_bound_box(float3 blo, float3 bhi, const BoundCtx &c, float *fast_m) {
     if (fast_m) *fast_m = 0.f;
-    const float q[6] = {node.lo[0] - c.p.x, node.hi[0] - c.p.x, node.lo[1] - c.p.y,
-                        node.hi[1] - c.p.y, node.lo[2] - c.p.z, node.hi[2] - c.p.z};
-    const CornerDots cn = corner_dots(c.n, q);
-    float cos_max = 0.f;
-    for (int i = 0; i < 8; i++)
-        if (cn.at(i) > 0.f) {
-            cos_max = 1.f;
-            break;
-        }
+    const float q[6] = {blo.x - c.p.x, bhi.x - c.p.x, blo.y - c.p.y, bhi.y - c.p.y, blo.z - c.p.z, bhi.z - c.p.z};
+    // some corner lies above the shading point's tangent plane
+    const float cos_max = corner_range(c.n, q).hi > 0.f ? 1.f : 0.f;
     if (cos_max <= 0.f) return 0.f;
     float maxp = 0.f;
     if (c.sl > 0.f) {
-        const Frame &hf = c.hf;
-        const CornerDots ct = corner_dots(hf.t, q), cb = corner_dots(hf.b, q), cz = corner_dots(hf.n, q);
-        float3 lo = f3(DR_INF), hi = f3(-DR_INF);
-        for (int i = 0; i < 8; i++) {
-            float3 v = f3(ct.at(i), cb.at(i), cz.at(i));  // to_local(hf, corner_i - p)
-            lo = f3(fminf(lo.x, v.x), fminf(lo.y, v.y), fminf(lo.z, v.z));
-            hi = f3(fmaxf(hi.x, v.x), fmaxf(hi.y, v.y), fmaxf(hi.z, v.z));
-        }
+        // the box in the frame around wi
+        const DotRange rx = corner_range(c.hf.t, q), ry = corner_range(c.hf.b, q), rz = corner_range(c.hf.n, q);
+        const float3 lo = f3(rx.lo, ry.lo, rz.lo), hi = f3(rx.hi, ry.hi, rz.hi);
         float cphi = 0.f;
         float hx = hi.x;
         if (hx > 0.f) cphi = hx / sqrtf(min_sq_bound(lo.y, hi.y) + hx * hx);
@@ -324,7 +315,11 @@ DEV_NOINLINE float bsdf_bound(const DevEdgeNode &node, const BoundCtx &c, float 
     return cos_max * (c.dl / DR_PI + c.sl * maxp);
 }
 
-
+DEV float3 node_lo(const DevEdgeNode &n) { return f3(n.lo[0], n.lo[1], n.lo[2]); }
+DEV float3 node_hi(const DevEdgeNode &n) { return f3(n.hi[0], n.hi[1], n.hi[2]); }
+DEV_NOINLINE float bsdf_bound(const DevEdgeNode &node, const BoundCtx &c, float *fast_m = nullptr) {
+    return bsdf_bound_box(node_lo(node), node_hi(node), c, fast_m);
+}
 
 // Whether the node's cone of normals, widened by the angle its bounding
 // sphere subtends from p, reaches the directions perpendicular to p - centre:
@@ -337,19 +332,21 @@ DEV_NOINLINE float bsdf_bound(const DevEdgeNode &node, const BoundCtx &c, float 
 // takes from the fast functions; it takes the same answer as the float
 // evaluation and leaves the rest to it, and also every |c| > 1 (rounding
 // can give that; acos is NaN there and the float evaluation answers false).
-DEV_NOINLINE bool contains_silhouette(const DevEdgeNode &node, float3 p) {
-    // bounding sphere as aabb.h:266-270: center (lo + hi) / 2, radius |hi - center|
-    float3 cs = f3((node.lo[0] + node.hi[0]) / 2.f, (node.lo[1] + node.hi[1]) / 2.f, (node.lo[2] + node.hi[2]) / 2.f);
-    float r = length(f3(node.hi[0], node.hi[1], node.hi[2]) - cs);
+// cs and r: the node's bounding sphere as aabb.h:266-270, center (lo + hi) / 2
+// and radius |hi - center|; sa and ca: the fast sine and cosine of the angle.
+DEV float3 sphere_center(float3 lo, float3 hi) {
+    return f3((lo.x + hi.x) / 2.f, (lo.y + hi.y) / 2.f, (lo.z + hi.z) / 2.f);
+}
+DEV bool cone_reaches_silhouette(float3 cs, float r, float3 axis, float a, float sa, float ca, float3 p) {
     float3 d = cs - p;
     float l = length(d);
     float vt = r / l;
     if (vt >= 1.f) return true;
     d = d / l;
-    const float c = dot(-d, f3(node.axis[0], node.axis[1], node.axis[2]));
-    const float a = node.angle, ac = fabsf(c);
+    const float c = dot(-d, axis);
+    const float ac = fabsf(c);
     if (a >= 0.f && a <= 1.5f && ac <= 1.f) {  // NaNs fall through to the float evaluation
-        const float k = filt_rsqrt(1.f + vt * vt), sa = filt_sin(a), ca = filt_cos(a);
+        const float k = filt_rsqrt(1.f + vt * vt);
         const float cos_r = (ca - vt * sa) * k, sin_r = (sa + vt * ca) * k;
         const float margin = 1e-5f;
         if (cos_r < -margin) return true;  // angle + atan(vt) > pi/2
@@ -360,8 +357,13 @@ DEV_NOINLINE bool contains_silhouette(const DevEdgeNode &node, float3 p) {
     }
     float va = dr_atanf(vt);
     float ang = dr_acosf(c);
-    float range = node.angle + va;
+    float range = a + va;
     return ang - range <= float(3.14159265358979323846 / 2.f) && ang + range >= float(3.14159265358979323846 / 2.f);
+}
+DEV_NOINLINE bool contains_silhouette(const DevEdgeNode &node, float3 p) {
+    const float3 hi = node_hi(node), cs = sphere_center(node_lo(node), hi);
+    return cone_reaches_silhouette(cs, length(hi - cs), f3(node.axis[0], node.axis[1], node.axis[2]), node.angle,
+                                   filt_sin(node.angle), filt_cos(node.angle), p);
 }
 
 // The float evaluation alone (checks of the filter).
@@ -379,14 +381,18 @@ HD bool contains_silhouette_exact(const DevEdgeNode &node, float3 p) {
     return ang - range <= float(3.14159265358979323846 / 2.f) && ang + range >= float(3.14159265358979323846 / 2.f);
 }
 
+DEV float box_importance(float3 lo, float3 hi, float total_length, float bb, float3 p) {
+    float3 c = f3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
+    return bb * total_length / length_sq(p - c);
+}
 DEV float node_importance(const DevEdgeNode &node, float bb, float3 p) {
-    float3 c = f3(0.5f * (node.lo[0] + node.hi[0]), 0.5f * (node.lo[1] + node.hi[1]), 0.5f * (node.lo[2] + node.hi[2]));
-    return bb * node.total_length / length_sq(p - c);
+    return box_importance(node_lo(node), node_hi(node), node.total_length, bb, p);
 }
 
-DEV bool node_inside(const DevEdgeNode &n, float3 p) {
-    return p.x >= n.lo[0] && p.x <= n.hi[0] && p.y >= n.lo[1] && p.y <= n.hi[1] && p.z >= n.lo[2] && p.z <= n.hi[2];
+DEV bool box_inside(float3 lo, float3 hi, float3 p) {
+    return p.x >= lo.x && p.x <= hi.x && p.y >= lo.y && p.y <= hi.y && p.z >= lo.z && p.z <= hi.z;
 }
+DEV bool node_inside(const DevEdgeNode &n, float3 p) { return box_inside(node_lo(n), node_hi(n), p); }
 
 // The learned edge proposal of one shading point (a project addition): 32
 // bf16 probabilities over directions from the point, in the shading frame:
@@ -406,9 +412,12 @@ DEV int dir_bin(const Frame &f, float3 d) {
     return band * 8 + oct;
 }
 // The proposal's weight of a node: its probability for the direction of the box centre.
-DEV float node_dir_weight(const uint16_t *q, const Frame &f, float3 p, const DevEdgeNode &n) {
-    float3 c = f3(0.5f * (n.lo[0] + n.hi[0]), 0.5f * (n.lo[1] + n.hi[1]), 0.5f * (n.lo[2] + n.hi[2]));
+DEV float box_dir_weight(const uint16_t *q, const Frame &f, float3 p, float3 lo, float3 hi) {
+    float3 c = f3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
     return bf16_bits_to_float(q[dir_bin(f, c - p)]);
+}
+DEV float node_dir_weight(const uint16_t *q, const Frame &f, float3 p, const DevEdgeNode &n) {
+    return box_dir_weight(q, f, p, node_lo(n), node_hi(n));
 }
 
 // Stochastic traversal of one edge tree in one mode (edge_tree.cpp:511-652):
@@ -441,13 +450,51 @@ template <bool PROP> HD EdgeItem<PROP> edge_item(int node, float bb, float c, fl
     return it;
 }
 
+// Whether filtered bounds (errors lm, rm; 0: exact) leave open what the
+// importances decide, the cutoff at 1e-10 and the cone tests' finiteness
+// check: the exact bounds are evaluated then.
+DEV bool filter_undecided(float il, float ir, float lm, float rm) {
+    const float m = 2.f * fmaxf(lm, rm) + 1e-6f, sum = il + ir;
+    return !(sum > 1e-10f * (1.f + m) || sum < 1e-10f * (1.f - m)) || !(il < 1e30f) || !(ir < 1e30f);
+}
+
+// How an interior node's two children share the walk (edge_tree.cpp:580-640):
+// whether the cone walk splits here, and each child's probability in the cone
+// walk (plc, prc) and in the all walk (pla, pra).  lcs, rcs: the children's
+// silhouette tests, lhc, rhc their cone tests, il, ir their importances.
+struct ChildShares {
+    bool cone_split;
+    float plc, prc, pla, pra;
+};
+DEV ChildShares child_shares(float il, float ir, bool lhc, bool rhc, bool lcs, bool rcs, bool all_split,
+                             float cos_angle) {
+    ChildShares c;
+    c.cone_split = all_split || (lhc && rhc && lcs && rcs && cos_angle > 0.95f);
+    const float ilc = lhc ? il : 0.f, irc = rhc ? ir : 0.f;
+    c.plc = c.prc = 0.f;
+    if (c.cone_split) {
+        c.plc = c.prc = 1.f;
+    } else if (ilc + irc > 1e-10f) {
+        c.plc = ilc / (ilc + irc);
+        c.prc = 1.f - c.plc;
+    }
+    if (all_split) {
+        c.pla = c.pra = 1.f;
+    } else {
+        c.pla = il / (il + ir);
+        c.pra = 1.f - c.pla;
+    }
+    return c;
+}
+
 // The children of an interior node as the traversal decides them
 // (edge_tree.cpp:560-650): both when the node splits, else the one drawn in
 // proportion to the importances.  Returns 0 when neither is walked (both
 // importances vanish), 1 for a split, 2 for a draw; push_l / push_r say which
 // children are walked (a child whose silhouette test fails or whose bound is
 // 0 is not), l_leaf / r_leaf whether they are leaves.  Shared by the
-// depth-first walk (EdgeWalk) and the level-by-level walk (k_edge_level).
+// depth-first walks (EdgeWalk); the warp walk (dr_edge_walk.cuh) decides a node
+// by the same rules, a child per lane.
 template <bool PROP> struct ChildPick {
     EdgeItem<PROP> left, right;
     bool push_l, push_r, l_leaf, r_leaf;
@@ -475,16 +522,11 @@ DEV int node_children(const DevEdgeNode *nodes, const BoundCtx &bc, const ConeSp
     float rbb = rcs ? bsdf_bound(R, bc, filt ? &rm : nullptr) : 0.f;
     float il = lcs ? node_importance(L, lbb, p) : 0.f;
     float ir = rcs ? node_importance(R, rbb, p) : 0.f;
-    if (lm > 0.f || rm > 0.f) {
-        // the cutoff and the cone tests' finiteness check as the exact
-        // bounds decide them: exact bounds where a filtered one could differ
-        const float m = 2.f * fmaxf(lm, rm) + 1e-6f, sum = il + ir;
-        if (!(sum > 1e-10f * (1.f + m) || sum < 1e-10f * (1.f - m)) || !(il < 1e30f) || !(ir < 1e30f)) {
-            lbb = lcs ? bsdf_bound(L, bc) : 0.f;
-            rbb = rcs ? bsdf_bound(R, bc) : 0.f;
-            il = lcs ? node_importance(L, lbb, p) : 0.f;
-            ir = rcs ? node_importance(R, rbb, p) : 0.f;
-        }
+    if ((lm > 0.f || rm > 0.f) && filter_undecided(il, ir, lm, rm)) {
+        lbb = lcs ? bsdf_bound(L, bc) : 0.f;
+        rbb = rcs ? bsdf_bound(R, bc) : 0.f;
+        il = lcs ? node_importance(L, lbb, p) : 0.f;
+        ir = rcs ? node_importance(R, rbb, p) : 0.f;
     }
     if (il + ir <= 1e-10f) return 0;
     // a node the cone walk cannot reach (cpmf 0) gives its children cpmf
@@ -492,22 +534,10 @@ DEV int node_children(const DevEdgeNode *nodes, const BoundCtx &bc, const ConeSp
     // finite: the all walk skips the tests there
     const bool cone_tests = CONE || it.cpmf != 0.f || !dr_isfinite(il) || !dr_isfinite(ir);
     bool lhc = cone_tests && box_cone(L.lo, L.hi, cone), rhc = cone_tests && box_cone(R.lo, R.hi, cone);
-    bool cone_split = all_split || (lhc && rhc && lcs && rcs && cone.cos_angle > 0.95f);
-    float ilc = lhc ? il : 0.f, irc = rhc ? ir : 0.f;
-    if (CONE && ilc + irc <= 1e-10f) return 0;
-    float plc = 0.f, prc = 0.f, pla = 0.f, pra = 0.f;
-    if (cone_split) {
-        plc = prc = 1.f;
-    } else if (ilc + irc > 1e-10f) {
-        plc = ilc / (ilc + irc);
-        prc = 1.f - plc;
-    }
-    if (all_split) {
-        pla = pra = 1.f;
-    } else {
-        pla = il / (il + ir);
-        pra = 1.f - pla;
-    }
+    if (CONE && (lhc ? il : 0.f) + (rhc ? ir : 0.f) <= 1e-10f) return 0;
+    const ChildShares sh = child_shares(il, ir, lhc, rhc, lcs, rcs, all_split, cone.cos_angle);
+    const bool cone_split = sh.cone_split;
+    const float plc = sh.plc, prc = sh.prc, pla = sh.pla, pra = sh.pra;
     // the proposal's choice (both children important, no split): importance
     // times the learned weight of the direction towards each child
     float pll = pla;
@@ -544,6 +574,35 @@ DEV int node_children(const DevEdgeNode *nodes, const BoundCtx &bc, const ConeSp
 }
 
 #define DR_NODE_MASK ((1 << 27) - 1)
+
+// The children of interior node `nid` packed side by side (DevScene::sil_box,
+// nrm_box, nrm_dir): box[4 nid + 2 c] = (lo, total length) and box[4 nid + 2 c
+// + 1] = (hi, child code) of child c (0 left, 1 right), 64 contiguous bytes per
+// parent; dir[4 nid + 2 c] = (cone axis, angle) and dir[4 nid + 2 c + 1] =
+// (bounding-sphere radius, the angle's fast sine and cosine, 0).  The code is
+// the child's node id for an interior child, DR_CHILD_LEAF | edge for a leaf
+// of one edge, DR_CHILD_LEAF | DR_CHILD_MANY | node id for a larger leaf.
+#define DR_CHILD_LEAF (1 << 30)
+#define DR_CHILD_MANY (1 << 29)
+DEV void pack_children(const DevEdgeNode *nodes, int nid, float4 *box, float4 *dir) {
+    if (nodes[nid].nprims > 0) return;  // a leaf has no children
+    for (int c = 0; c < 2; c++) {
+        const int ci = c ? nodes[nid].offset : nid + 1;
+        const DevEdgeNode &n = nodes[ci];
+        int code = ci;
+        if (n.nprims == 1) code = DR_CHILD_LEAF | n.offset;
+        else if (n.nprims > 1) code = DR_CHILD_LEAF | DR_CHILD_MANY | ci;
+        float4 *b = box + 4 * (size_t)nid + 2 * c;
+        b[0].x = n.lo[0], b[0].y = n.lo[1], b[0].z = n.lo[2], b[0].w = n.total_length;
+        b[1].x = n.hi[0], b[1].y = n.hi[1], b[1].z = n.hi[2], b[1].w = dr_i2f(code);
+        if (!dir) continue;
+        float4 *d = dir + 4 * (size_t)nid + 2 * c;
+        const float3 hi = node_hi(n);
+        d[0].x = n.axis[0], d[0].y = n.axis[1], d[0].z = n.axis[2], d[0].w = n.angle;
+        d[1].x = length(hi - sphere_center(node_lo(n), hi));
+        d[1].y = filt_sin(n.angle), d[1].z = filt_cos(n.angle), d[1].w = 0.f;
+    }
+}
 
 // The walk of one tree in one mode as a resumable state: start() pushes the
 // root or a handed-on subtree, step() takes one node off the stack.  A kernel

@@ -12,7 +12,7 @@
 // mark synchronizes the stream and remembers the first kernel that failed.
 struct StageTimer {
     // a streamed edge stage marks its kernels once per chunk of points, the
-    // level walk's two once per level
+    // walk once per round
     static const int kMax = 4096;
     bool on = false;
     bool sync = false;
@@ -85,6 +85,10 @@ cudaError_t dr_launch_forward(const DevScene &s, int W, int H, int spp, int B, u
 // Backward pass (dr_backward.cu).
 // Queue counters on the device.  They are 64-bit and keep counting past a
 // queue's capacity, so the host learns how many entries a launch needed.
+// Rounds of the warp walk (k_edge_walk) and the size of the packets of pending
+// nodes it hands from one to the next.
+#define DR_WALK_ROUNDS 6
+#define DR_WALK_PACKET_BYTES 544
 struct BackwardCounters {
     unsigned long long points;  // shading points appended by k_backward_paths
     unsigned long long items;   // edge items appended by the last k_edge_traverse
@@ -105,11 +109,9 @@ struct BackwardCounters {
     // subtrees handed on between rounds of k_edge_tasks (two queues, used in
     // turn) and their total
     unsigned long long handed[2], handed_total;
-    // leaves the level walk's launch queued for k_edge_leaves; the nodes it
-    // queued for the next level, per class (front and back half of the
-    // queue, two queues used in turn); subtrees a full queue left to a lane's
-    // depth-first walk
-    unsigned long long leaf_n, level_n[2][2], spilled;
+    // k_edge_walk's rounds: the next batch each round takes, and the packets
+    // it handed on
+    unsigned long long walk_next[DR_WALK_ROUNDS], walk_n[DR_WALK_ROUNDS];
 };
 
 // A view of a batched multi-view backward call: what the edge stage needs of
@@ -164,18 +166,18 @@ struct BackwardWorkspace {
     // its shallowest pending subtree on, and launches (rounds) per chunk of
     // points (the scene's tuning, dr_scene_set_tuning)
     int hand_steps = 64, task_rounds = 3;
-    // the level-by-level walk of the subtrees (level_walk != 0; otherwise
-    // k_edge_tasks walks each depth first): every point's walk context
-    // ([cap_points][DR_CTX_F4] float4, k_walk_ctx) and the queue of the
-    // leaves each level reached (cap_leaves entries); the levels' own queues
-    // are `tasks` and `tasks2`, used in turn
-    int level_walk = 1;
+    // every point's walk context ([cap_points][DR_CTX_F4] float4, k_walk_ctx)
+    // where a warp walks a batch of points (k_edge_walk); null: the point
+    // walks of k_edge_traverse, or with `tasks` of k_edge_expand and
+    // k_edge_tasks
     float4 *walk_ctx;
+    // [2][cap_packets] x DR_WALK_PACKET_BYTES: pending nodes handed from one
+    // round of k_edge_walk to the next (two queues, used in turn)
+    void *packets;
+    long long cap_packets;
     // [cap_points][DR_LCTX_F4] each point's line-sample setup (k_line_ctx;
     // null: k_edge_line sets it up per edge)
     float4 *line_ctx;
-    EdgeTask *leafq;
-    long long cap_leaves;
     // per view of a batched multi-view call (null: the call's own settings);
     // each point's settings are views[point.view]
     const ViewParams *views;
@@ -219,6 +221,8 @@ cudaError_t dr_launch_edge_traverse(const DevScene &s, uint64_t seed, const Back
                                     cudaStream_t st, int *launches, StageTimer *timer);
 // The silhouette-test records of n tree edges (dr_edges.cuh: edge_record).
 cudaError_t dr_launch_edge_records(const DevScene &s, const DevEdge *edges, int n, EdgeRec *out, cudaStream_t st);
+// Each interior node's children side by side (dr_edges.cuh: pack_children).
+cudaError_t dr_launch_edge_children(const DevEdgeNode *nodes, int n, float4 *box, float4 *dir, cudaStream_t st);
 // out[b] = edges sampled by points [b P / nb, (b + 1) P / nb) (ws.pt_items)
 cudaError_t dr_launch_item_buckets(const int *pt_items, long long P, int nb, unsigned long long *out,
                                    cudaStream_t st);

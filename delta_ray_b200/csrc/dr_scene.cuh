@@ -137,6 +137,9 @@ struct DevScene {
     const DevEdge *nrm_edges;
     int num_nrm_nodes;
     const EdgeRec *sil_rec, *nrm_rec;  // per tree edge, in the trees' edge order
+    // each interior node's children side by side (dr_edges.cuh: pack_children),
+    // 4 float4 per node id; built for trees the warp walk reads, else null
+    const float4 *sil_box, *nrm_box, *nrm_dir;
     const float *ltc;      // 128*128 row-major 3x3, Blinn-Phong lobes
     const float *ltc_ggx;  // the same for GGX lobes
     int grad_total;

@@ -272,9 +272,9 @@ class Scene:
         items, line samples passed to the ray stage (for large meshes: those
         whose rays hit one of the edge's faces), shaded samples, subtree tasks,
         first-stage items,
-        node visits of the point walks and of the subtree walks, candidates of
-        the ray stage (samples that passed its connectivity test), subtrees
-        walked depth first after a full level queue."""
+        node visits of the point walks and of the large trees' walks,
+        candidates of the ray stage (samples that passed its connectivity
+        test), and 0 (reserved)."""
         w = (C.c_int64 * 10)()
         _lib.check(_lib.lib().dr_scene_last_work(self.handle, w, 10))
         keys = ("points", "items", "survivors", "shaded", "tasks", "items_first_stage", "visits_walk",

@@ -278,12 +278,12 @@ DR_API dr_status dr_render_backward_noalloc(dr_scene *scene, const dr_render_des
 DR_API dr_status dr_set_item_queue_limit(int64_t items);
 
 /* A scene's queue settings for its backward calls (no counterpart in the
- * reference, whose CPU renderer has no work queues).  Large edge trees are
- * walked in two stages: each point's walk down to 8 levels below the roots,
- * then the subtrees there.
- *   depth_first: 0 (the default) walks those subtrees level by level, one
- *     launch per level over every subtree's nodes of that level; 1 walks
- *     each subtree depth first, one lane per subtree;
+ * reference, whose CPU renderer has no work queues).
+ *   depth_first: how large edge trees are walked: 0 (the default) by warps,
+ *     each walking a batch of points with its pending nodes in shared memory
+ *     and handing long walks on in rounds; 1 in two stages, each point's walk
+ *     down to 8 levels below the roots, then the subtrees there depth first,
+ *     one lane per subtree;
  *   hand_steps: with depth_first, the node steps a subtree walk takes before
  *     it hands its shallowest pending subtree on to the next round
  *     (1..4096; default 64);
@@ -380,14 +380,13 @@ DR_API dr_status dr_scene_edge_data(const dr_scene *scene, int what, void *out_h
  * of its kernels; no counterpart in the reference): counts[0] shading points,
  * [1] sampled edges, [2] line samples kept for their rays (in scenes
  * traced through the LBVH: those whose rays hit one of the edge's faces),
- * [3] samples kept for shading, [4] subtrees walked by the second traversal
- * stage (handed on by the first stage, and with the depth-first walk between
- * its rounds),
+ * [3] samples kept for shading, [4] walks of large trees begun (two per
+ * point); with the depth-first walk, the subtrees handed on by its first stage
+ * and between its rounds,
  * [5] edges sampled by the first stage (all, when the traversal runs in one
  * stage), [6] edge-tree nodes visited by the point walks, [7] nodes
- * visited by the subtree walks, [8] line samples whose connectivity test
- * passed (candidates of the ray stage), [9] subtrees the level walk left to
- * a lane's depth-first walk because a level's queue was full.  Up to n of
+ * visited by the walks of large trees, [8] line samples whose connectivity test
+ * passed (candidates of the ray stage), [9] 0 (reserved).  Up to n of
  * them are written. */
 DR_API dr_status dr_scene_last_work(const dr_scene *scene, int64_t *counts, int n);
 
