@@ -410,8 +410,9 @@ void build_edge_records(dr_scene *sc, cudaStream_t st) {
     sc->ds.sil_box = sc->ds.nrm_box = sc->ds.nrm_dir = nullptr;
     if (split) {
         float4 *k = reinterpret_cast<float4 *>((char *)sc->edge_recs.p + rec_bytes);
-        check_cuda(dr_launch_edge_children(sc->ds.sil_nodes, sc->ds.num_sil_nodes, k, nullptr, st), "edge children");
-        check_cuda(dr_launch_edge_children(sc->ds.nrm_nodes, sc->ds.num_nrm_nodes, k + s4, k + s4 + n4, st),
+        check_cuda(dr_launch_edge_children(sc->ds.sil_nodes, r, sc->ds.num_sil_nodes, k, nullptr, st),
+                   "edge children");
+        check_cuda(dr_launch_edge_children(sc->ds.nrm_nodes, r + ns, sc->ds.num_nrm_nodes, k + s4, k + s4 + n4, st),
                    "edge children");
         sc->last_launches += 2;
         sc->ds.sil_box = k;

@@ -649,8 +649,7 @@ DEV bool item_line(const DevScene &s, const PointRecord &pt, int tree, int ei, u
     Rng prng;
     prng.init(seed, kStreamEdgePoint, pt.sid, (uint32_t)pt.bounce);
     EdgeSample es = draw_edge(prng);
-    const DevEdge &edge = tree ? s.nrm_edges[ei] : s.sil_edges[ei];
-    return edge_line_sample<EXT>(s, es, edge, pt.wi, pt.tri, pt.surface(), el, (tree ? s.nrm_rec : s.sil_rec) + ei);
+    return edge_line_sample<EXT>(s, es, (tree ? s.nrm_rec : s.sil_rec) + ei, pt.wi, pt.tri, pt.surface(), el);
 }
 
 // The item's shading from its line sample; as eval_item.  `hits` (may be
@@ -685,7 +684,7 @@ DEV float3 item_shade(const DevScene &s, const PointRecord &pt, int tree, int ei
     else
         er = hits ? edge_shade_hits<MAYBE_GI>(s, el, edge, els, irng, B - pt.bounce - 1, pt.wi, pt.tri, pt.surface(),
                                               weight, pt.d_color, B == 1, *hits)
-                  : edge_shade_sample<MAYBE_GI>(s, el, edge, els, irng, B - pt.bounce - 1, pt.wi, pt.tri,
+                  : edge_shade_sample<MAYBE_GI>(s, el, edge, (tree ? s.nrm_rec : s.sil_rec) + ei, els, irng, B - pt.bounce - 1, pt.wi, pt.tri,
                                                 pt.surface(), weight, pt.d_color, B == 1);
     if (EXT && mag) *mag = abs_sum(er.dv0) + abs_sum(er.dv1);
     if (!is_zero(er.dv0) || !is_zero(er.dv1)) {

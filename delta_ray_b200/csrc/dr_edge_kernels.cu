@@ -21,9 +21,9 @@ namespace cg = cooperative_groups;
 #endif
 // and of the line and side-radiance kernels (a sweep at the 640x480
 // heightfield: radiance 3 / 4 / 6 / 8 blocks 264 / 249 / 223 / 234 ms per
-// step; line 4 and 6 the same; connect 6 / 8 / 10: 458 / 436 / 516)
+// step)
 #ifndef DR_LINE_BLOCKS
-#define DR_LINE_BLOCKS 4
+#define DR_LINE_BLOCKS 7
 #endif
 #ifndef DR_RADIANCE_BLOCKS
 #define DR_RADIANCE_BLOCKS 6
@@ -365,169 +365,9 @@ __device__ __forceinline__ void finish_item(const DevScene &s, const BackwardWor
 //
 // EXT: DR_FLAG_EDGE_LOBE_MIS or proposal training in use; GI: max_bounces > 1
 // (the shade calls of the two sides); the launcher picks the variant.
-// Each point's line-sample setup (line_setup: the point's edge draw, lobe
-// pick and LTC transforms), the same for all of its thousands of edges: the
-// line kernel reads it instead of setting it up per edge.  Layout, float4:
-// 0-2 minv and 3-5 m with the lobe's pick probability, the draw's u, ok and
-// the point's position in the last words of the two matrices' rows.
-__global__ void __launch_bounds__(128, 8) k_line_ctx(DevScene s, uint64_t seed, BackwardWorkspace ws) {
-    const long long n = min(min((long long)ws.counters->points, ws.cap_points), ws.pt_end);
-    for (long long p = ws.pt_begin + (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-         p += (long long)gridDim.x * blockDim.x) {
-        PointRecord pt;
-        pt.load(ws.pt + (size_t)p * DR_PT_WORDS);
-        Rng prng;
-        prng.init(point_seed(ws, pt.view, seed), kStreamEdgePoint, pt.sid, (uint32_t)pt.bounce);
-        const EdgeSample es = draw_edge(prng);
-        const LineSetup ls = line_setup(s, es, pt.wi, pt.tri, pt.surface());
-        const float *a = ls.minv.m, *b = ls.m.m;
-        float4 *o = ws.line_ctx + (size_t)p * DR_LCTX_F4;
-        o[0] = make_float4(a[0], a[1], a[2], a[3]);
-        o[1] = make_float4(a[4], a[5], a[6], a[7]);
-        o[2] = make_float4(a[8], b[0], b[1], b[2]);
-        o[3] = make_float4(b[3], b[4], b[5], b[6]);
-        o[4] = make_float4(b[7], b[8], ls.mpmf, es.u);
-        o[5] = make_float4(ls.ok ? 1.f : 0.f, pt.p.x, pt.p.y, pt.p.z);
-    }
-}
+#include "dr_edge_line.cuh"
 
-template <bool EXT>
-__global__ void __launch_bounds__(128, DR_LINE_BLOCKS) k_edge_line(DevScene s, uint64_t seed, BackwardWorkspace ws) {
-    long long n = (long long)min(ws.counters->items, (unsigned long long)ws.cap_items);
-    long long stride = (long long)gridDim.x * blockDim.x;
-    // warp-uniform loop: the survivor append is warp-aggregated
-    for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += stride) {
-        long long i = base + (threadIdx.x & 31);
-        EdgeLine el;
-        bool ok = false;
-        if (i < n) {
-            int4 it = ws.items[i];
-            const int tree = it.y >> 30, ei = it.y & ((1 << 30) - 1);
-            PointRecord pt;
-            if (!EXT && ws.line_ctx) {
-                const float4 *c = ws.line_ctx + (size_t)it.x * DR_LCTX_F4;
-                const float4 c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3], c4 = c[4], c5 = c[5];
-                LineSetup ls;
-                const float ma[9] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w, c2.x};
-                const float mb[9] = {c2.y, c2.z, c2.w, c3.x, c3.y, c3.z, c3.w, c4.x, c4.y};
-                for (int k = 0; k < 9; k++) {
-                    ls.minv.m[k] = ma[k];
-                    ls.m.m[k] = mb[k];
-                }
-                ls.mpmf = c4.z;
-                EdgeSample es;
-                es.u = c4.w;
-                es.bsdf_component = 0.f;  // the lobe pick is in the setup
-                pt.p = f3(c5.y, c5.z, c5.w);
-                const DevEdge &edge = tree ? s.nrm_edges[ei] : s.sil_edges[ei];
-                SurfacePoint unused;
-                ok = c5.x != 0.f && line_sample_from<false>(s, ls, es, edge, pt.p, unused, f3(0.f), el,
-                                                             (tree ? s.nrm_rec : s.sil_rec) + ei);
-            } else {
-                pt.load(ws.pt + (size_t)it.x * DR_PT_WORDS);
-                ok = item_line<EXT>(s, pt, tree, ei, point_seed(ws, pt.view, seed), el);
-            }
-            if (ok) {
-                // the connectivity test's first part: a sample neither of whose
-                // rays hits one of the edge's faces is connected on no side
-                // (three in four samples of a large mesh end here)
-                const DevEdge &edge = tree ? s.nrm_edges[ei] : s.sil_edges[ei];
-                float3 sdir, rdir, ldir;
-                edge_side_dirs(el, edge_v0(s, edge), edge_v1(s, edge), pt.p, sdir, rdir, ldir);
-                Hit fr, fl;
-                hit_faces_pair(s, edge, pt.p, rdir, ldir, 1e-3f, fr, fl);
-                ok = fr.tri >= 0 || fl.tri >= 0;
-            }
-        }
-        __syncwarp();
-        unsigned long long slot = warp_reserve(&ws.counters->survivors, ok ? 1 : 0);
-        if (ok) {
-            ws.survivors[2 * slot] = make_float4(__int_as_float((int)i), el.sample_p.x, el.sample_p.y, el.sample_p.z);
-            ws.survivors[2 * slot + 1] = make_float4(el.mwt.x, el.mwt.y, el.mwt.z, el.q);
-        }
-    }
-}
-
-// The ray stage of an LBVH scene in two kernels.  k_edge_connect decides
-// each line sample's connectivity (the edge's faces and one or two bounded
-// occlusion walks; most samples end here) and queues the few that go on;
-// k_edge_pairs traces the other side's closest hit of those and runs the
-// remaining tests.  Walk lengths vary widely, so both fetch their work one
-// item per lane (a lane takes the next as soon as it is done) rather than a
-// warp's worth at a time.
-__global__ void __launch_bounds__(128, DR_CONNECT_BLOCKS) k_edge_connect(DevScene s, BackwardWorkspace ws) {
-    const long long n = (long long)min(ws.counters->survivors, (unsigned long long)ws.cap_items);
-    // A state machine per lane, stepped by the whole warp.  When at least
-    // half the warp has no walk (or none has), those lanes take line samples
-    // together (a sample's setup and face tests cost about ten walk steps)
-    // until each has one that needs an occlusion walk; otherwise every
-    // walking lane takes one node, at the same point of the code.  (Lanes
-    // that ran their walks to the end before taking the next sample, and
-    // lanes that took one as soon as they were idle, left the warp split
-    // into groups issuing on their own: 5.1 and 3.8 of 32 lanes active.)
-    long long k = 0;
-    int phase = 0;  // 0 no walk, 1 walking the right ray, 2 walking the left ray
-    bool more = true, cr = false;
-    float3 p = f3(0.f), rdir = f3(0.f), ldir = f3(0.f);
-    Hit fr, fl;
-    fr.tri = fl.tri = -1;
-    fr.t = fl.t = 0.f;
-    BeforeWalk w;
-    auto candidate = [&](int side, int face) {
-        const long long j = next_task(&ws.counters->cands);
-        ws.hits[j] = make_int4((int)k, face, side, 0);
-    };
-    while (true) {
-        const unsigned walking = __ballot_sync(0xffffffffu, phase != 0);
-        const unsigned idle = __ballot_sync(0xffffffffu, phase == 0 && more);
-        if (walking == 0 && idle == 0) break;  // every lane's queue has ended
-        const bool fetch = idle != 0 && (__popc(idle) >= 16 || walking == 0);
-        while (fetch && phase == 0 && more) {
-            k = next_task(&ws.counters->ray_next);
-            if (k >= n) {
-                more = false;
-                break;
-            }
-            const float4 a = ws.survivors[2 * k];
-            const int4 it = ws.items[__float_as_int(a.x)];
-            const float *pw = ws.pt + (size_t)it.x * DR_PT_WORDS;  // the point's position: words 0-2
-            const int tree = it.y >> 30, ei = it.y & ((1 << 30) - 1);
-            const DevEdge &edge = tree ? s.nrm_edges[ei] : s.sil_edges[ei];
-            p = f3(pw[0], pw[1], pw[2]);
-            EdgeLine el;
-            el.sample_p = f3(a.y, a.z, a.w);
-            float3 sdir;
-            edge_side_dirs(el, edge_v0(s, edge), edge_v1(s, edge), p, sdir, rdir, ldir);
-            // the connectivity test of edge_connect_bvh, its walks stepped below
-            hit_faces_pair(s, edge, p, rdir, ldir, 1e-3f, fr, fl);
-            if (fr.tri >= 0) {
-                w.begin(s.bvh_root, p, rdir, 1e-3f, fr.t, fr.tri);
-                phase = 1;
-            } else if (fl.tri >= 0) {
-                cr = false;
-                w.begin(s.bvh_root, p, ldir, 1e-3f, fl.t, fl.tri);
-                phase = 2;
-            }
-        }
-        if (fetch || phase == 0) continue;
-        const int r = w.step(s.bvh_nodes, s.bvh_wide, s.bvh_tris);
-        if (r == 0) continue;
-        if (phase == 1) {
-            cr = r == 2;  // no triangle ahead of the right face hit
-            if (fl.tri >= 0) {  // the left side decides (both connected, or neither, ends the sample)
-                w.begin(s.bvh_root, p, ldir, 1e-3f, fl.t, fl.tri);
-                phase = 2;
-            } else {
-                if (cr) candidate(0, fr.tri);  // the left ray hits no face: not connected
-                phase = 0;
-            }
-        } else {
-            const bool cl = r == 2;
-            if (cr != cl) candidate(cr ? 0 : 1, cr ? fr.tri : fl.tri);
-            phase = 0;
-        }
-    }
-}
+#include "dr_edge_connect.cuh"
 
 template <bool DIRECT>
 __global__ void __launch_bounds__(128, 4) k_edge_pairs(DevScene s, BackwardWorkspace ws) {
@@ -577,7 +417,7 @@ __global__ void __launch_bounds__(128, 8) k_edge_line_rays(DevScene s, uint64_t 
             ok = item_line<EXT>(s, pt, tree, ei, point_seed(ws, pt.view, seed), el);
             if (ok) {
                 const DevEdge &edge = tree ? s.nrm_edges[ei] : s.sil_edges[ei];
-                ok = edge_rays(s, el, edge, pt.tri, pt.p, DIRECT, eh);
+                ok = edge_rays(s, el, edge, (tree ? s.nrm_rec : s.sil_rec) + ei, pt.tri, pt.p, DIRECT, eh);
             }
         }
         __syncwarp();
@@ -703,14 +543,15 @@ cudaError_t dr_launch_edge_records(const DevScene &s, const DevEdge *edges, int 
     return cudaGetLastError();
 }
 
-__global__ void k_edge_children(const DevEdgeNode *nodes, int n, float4 *box, float4 *dir) {
+__global__ void k_edge_children(const DevEdgeNode *nodes, const EdgeRec *recs, int n, float4 *box, float4 *dir) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) pack_children(nodes, i, box, dir);
+    if (i < n) pack_children(nodes, recs, i, box, dir);
 }
 
-cudaError_t dr_launch_edge_children(const DevEdgeNode *nodes, int n, float4 *box, float4 *dir, cudaStream_t st) {
+cudaError_t dr_launch_edge_children(const DevEdgeNode *nodes, const EdgeRec *recs, int n, float4 *box, float4 *dir,
+                                    cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    k_edge_children<<<(n + 255) / 256, 256, 0, st>>>(nodes, n, box, dir);
+    k_edge_children<<<(n + 255) / 256, 256, 0, st>>>(nodes, recs, n, box, dir);
     return cudaGetLastError();
 }
 
@@ -826,15 +667,21 @@ cudaError_t dr_launch_edge_eval(const DevScene &s, int W, int H, int spp, int B,
         timer->mark(st, "k_edge_line_rays");
         *launches -= 1;
     } else {
-        if (!ext && ws.line_ctx) {
-            k_line_ctx<<<grid, 128, 0, st>>>(s, seed, ws);
+        if (ws.line_ctx) {
+            const bool mis = s.edge_lobe_mis != 0;
+            if (mis) k_line_ctx<true><<<grid, 128, 0, st>>>(s, seed, ws);
+            else k_line_ctx<false><<<grid, 128, 0, st>>>(s, seed, ws);
             timer->mark(st, "k_line_ctx");
+            if (mis) k_edge_line<true><<<num_sms * DR_LINE_BLOCKS, 128, 0, st>>>(s, ws);
+            else k_edge_line<false><<<num_sms * DR_LINE_BLOCKS, 128, 0, st>>>(s, ws);
             *launches += 1;
+        } else if (ext) {
+            k_edge_line_point<true><<<grid, 128, 0, st>>>(s, seed, ws);
+        } else {
+            k_edge_line_point<false><<<grid, 128, 0, st>>>(s, seed, ws);
         }
-        if (ext) k_edge_line<true><<<grid, 128, 0, st>>>(s, seed, ws);
-        else k_edge_line<false><<<grid, 128, 0, st>>>(s, seed, ws);
         timer->mark(st, "k_edge_line");
-        k_edge_connect<<<grid, 128, 0, st>>>(s, ws);
+        k_edge_connect<<<num_sms * DR_CONNECT_BLOCKS, 128, 0, st>>>(s, ws);
         timer->mark(st, "k_edge_connect");
         if (B > 1) k_edge_pairs<false><<<grid, 128, 0, st>>>(s, ws);
         else k_edge_pairs<true><<<grid, 128, 0, st>>>(s, ws);
@@ -923,7 +770,9 @@ cudaError_t dr_preload_edge_kernels() {
         (const void *)k_edge_walk<false>, (const void *)k_edge_walk<true>,
         (const void *)k_edge_line_rays<false, false>, (const void *)k_edge_line_rays<false, true>,
         (const void *)k_edge_line_rays<true, false>, (const void *)k_edge_line_rays<true, true>,
-        (const void *)k_edge_line<false>, (const void *)k_edge_line<true>, (const void *)k_line_ctx,
+        (const void *)k_edge_line<false>, (const void *)k_edge_line<true>,
+        (const void *)k_edge_line_point<false>, (const void *)k_edge_line_point<true>,
+        (const void *)k_line_ctx<false>, (const void *)k_line_ctx<true>,
         (const void *)k_edge_connect, (const void *)k_edge_pairs<false>, (const void *)k_edge_pairs<true>,
         (const void *)k_edge_radiance,
         (const void *)k_edge_shade<false, false, false>, (const void *)k_edge_shade<false, true, false>,
@@ -937,8 +786,10 @@ cudaError_t dr_preload_edge_kernels() {
         const cudaError_t e = cudaFuncGetAttributes(&a, f);
         if (e != cudaSuccess) return e;
     }
-    // the walk's resident blocks need most of the SM's shared memory
-    for (const void *f : {(const void *)k_edge_walk<false>, (const void *)k_edge_walk<true>}) {
+    // the walk's and the line kernel's resident blocks need most of the SM's
+    // shared memory
+    for (const void *f : {(const void *)k_edge_walk<false>, (const void *)k_edge_walk<true>,
+                          (const void *)k_edge_line<false>, (const void *)k_edge_line<true>}) {
         const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
                                                    cudaSharedmemCarveoutMaxShared);
         if (e != cudaSuccess) return e;

@@ -430,10 +430,13 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
                 const float denom = ccpmf * ccpmf + a * a;
                 w = cone_mode ? ccpmf / denom : a / denom;
             }
-            const bool keep = leaf && w != 0.f, node = push && !leaf;
+            // an edge that is a silhouette from everywhere is an item at once;
+            // the others wait for their test
+            const bool sure = leaf && w != 0.f && (child & DR_CHILD_SURE) && !(PROP && ws.train_targets);
+            const bool keep = leaf && w != 0.f && !sure, node = push && !leaf;
             const bool to0 = node && (cone_mode || ccpmf != 0.f), to1 = node && !to0;
             const unsigned m0 = __ballot_sync(full, to0), m1 = __ballot_sync(full, to1),
-                           ml = __ballot_sync(full, keep);
+                           ml = __ballot_sync(full, keep), ms = __ballot_sync(full, sure);
             visits += __popc(__ballot_sync(full, leaf));
             const unsigned tag = code & (15u << 27);  // slot and mode
             if (node) {
@@ -452,11 +455,19 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
                 sh.leaf[nl + __popc(ml & below)] =
                     make_uint2(tag | (unsigned)(child & DR_NODE_MASK) | ((child & DR_CHILD_MANY) ? 1u << 31 : 0u),
                                __float_as_uint(w));
+            } else if (sure) {
+                const int at = ni + __popc(ms & below);
+                sh.item[at] = make_uint2(tag | (unsigned)(child & DR_NODE_MASK), __float_as_uint(w));
+                if constexpr (PROP) sh.item_code[at] = 0;
+                if (nb > 1) atomicAdd(&sh.cnt[slot], 1);
             }
+            if (nb == 1 && lane == 0) sh.cnt[0] += __popc(ms);
+            ni += __popc(ms);
             n0 += __popc(m0);
             n1 += __popc(m1);
             nl += __popc(ml);
             __syncwarp();
+            if (ni > DR_WALK_ITEMS - 32) flush();
             if (nl >= 32) leaves(32);
         }
         if (nl > 0) leaves(nl);

@@ -8,7 +8,7 @@
 //                           explicit stack that keeps the same depth-first
 //                           order (left child first), so random draws are
 //                           consumed in the reference's order
-//   shading_edge_sample     delta_ray.cpp:45-365 (LTC line sampling, two rays
+//   line_sample_from, edge_rays, edge_shade_hits  delta_ray.cpp:45-365 (LTC line sampling, two rays
 //                           straddling the edge, dp/dv0/dv1)
 //   primary_edge_sample     delta_ray.cpp:377-557 (screen-space boundary
 //                           term, forward differences to world space)
@@ -40,24 +40,42 @@ DEV bool is_silhouette(const DevScene &s, float3 p, const DevEdge &e) {
     return (f0 && !f1) || (!f0 && f1);
 }
 
-// The silhouette test's record of an edge (see EdgeRec): the same operands
-// is_silhouette computes, so that is_silhouette_rec gives its answer.
+// An edge's record (see EdgeRec): the same operands is_silhouette computes, so
+// that is_silhouette_rec gives its answer, and those of the faces' hit test.
 DEV EdgeRec edge_record(const DevScene &s, const DevEdge &e) {
     EdgeRec r;
     const bool always = !s.shapes[e.shape].has_n || e.f0 == -1 || e.f1 == -1;
     float3 v0 = edge_v0(s, e), v1 = edge_v1(s, e), a = v0, b = v1, n0 = f3(0.f), n1 = f3(0.f);
+    if (e.f0 >= 0) a = non_shared_vertex(s, e, e.f0);
+    if (e.f1 >= 0) b = non_shared_vertex(s, e, e.f1);
     if (!always) {
-        a = non_shared_vertex(s, e, e.f0);
-        b = non_shared_vertex(s, e, e.f1);
         n0 = normalize(cross(v0 - a, v1 - a));
         n1 = normalize(cross(v1 - b, v0 - b));
+    }
+    int corners = 0, g[2] = {-1, -1};
+    for (int k = 0; k < 2; k++) {
+        const int f = k ? e.f1 : e.f0;
+        if (f < 0) continue;
+        g[k] = s.shapes[e.shape].tri_off + f;
+        const int4 t = s.tri[g[k]];
+        const int off = s.shapes[e.shape].vtx_off, v[3] = {t.x - off, t.y - off, t.z - off};
+        for (int i = 0; i < 3; i++) corners |= (v[i] == e.v0 ? 0 : (v[i] == e.v1 ? 1 : 2)) << (6 * k + 2 * i);
     }
     r.r[0].x = v0.x, r.r[0].y = v0.y, r.r[0].z = v0.z, r.r[0].w = n0.x;
     r.r[1].x = v1.x, r.r[1].y = v1.y, r.r[1].z = v1.z, r.r[1].w = n0.y;
     r.r[2].x = a.x, r.r[2].y = a.y, r.r[2].z = a.z, r.r[2].w = n0.z;
     r.r[3].x = b.x, r.r[3].y = b.y, r.r[3].z = b.z, r.r[3].w = n1.x;
-    r.r[4].x = n1.y, r.r[4].y = n1.z, r.r[4].z = always ? 1.f : 0.f, r.r[4].w = 0.f;
+    r.r[4].x = n1.y, r.r[4].y = n1.z, r.r[4].z = always ? 1.f : 0.f, r.r[4].w = dr_i2f(corners);
+    r.r[5].x = dr_i2f(g[0]), r.r[5].y = dr_i2f(g[1]), r.r[5].z = 0.f, r.r[5].w = 0.f;
     return r;
+}
+DEV float3 rec_v0(const EdgeRec *rec) {
+    const float4 q = dr_ldg(&rec->r[0]);
+    return f3(q.x, q.y, q.z);
+}
+DEV float3 rec_v1(const EdgeRec *rec) {
+    const float4 q = dr_ldg(&rec->r[1]);
+    return f3(q.x, q.y, q.z);
 }
 
 DEV bool is_silhouette_rec(const EdgeRec *rec, float3 p) {
@@ -581,16 +599,18 @@ DEV int node_children(const DevEdgeNode *nodes, const BoundCtx &bc, const ConeSp
 // parent; dir[4 nid + 2 c] = (cone axis, angle) and dir[4 nid + 2 c + 1] =
 // (bounding-sphere radius, the angle's fast sine and cosine, 0).  The code is
 // the child's node id for an interior child, DR_CHILD_LEAF | edge for a leaf
-// of one edge, DR_CHILD_LEAF | DR_CHILD_MANY | node id for a larger leaf.
+// of one edge, with DR_CHILD_SURE if it is a silhouette from everywhere,
+// DR_CHILD_LEAF | DR_CHILD_MANY | node id for a larger leaf.
 #define DR_CHILD_LEAF (1 << 30)
 #define DR_CHILD_MANY (1 << 29)
-DEV void pack_children(const DevEdgeNode *nodes, int nid, float4 *box, float4 *dir) {
+#define DR_CHILD_SURE (1 << 28)
+DEV void pack_children(const DevEdgeNode *nodes, const EdgeRec *recs, int nid, float4 *box, float4 *dir) {
     if (nodes[nid].nprims > 0) return;  // a leaf has no children
     for (int c = 0; c < 2; c++) {
         const int ci = c ? nodes[nid].offset : nid + 1;
         const DevEdgeNode &n = nodes[ci];
         int code = ci;
-        if (n.nprims == 1) code = DR_CHILD_LEAF | n.offset;
+        if (n.nprims == 1) code = DR_CHILD_LEAF | n.offset | (recs[n.offset].r[4].z != 0.f ? DR_CHILD_SURE : 0);
         else if (n.nprims > 1) code = DR_CHILD_LEAF | DR_CHILD_MANY | ci;
         float4 *b = box + 4 * (size_t)nid + 2 * c;
         b[0].x = n.lo[0], b[0].y = n.lo[1], b[0].z = n.lo[2], b[0].w = n.total_length;
@@ -892,20 +912,22 @@ DEV_NOINLINE float lobe_line_density(const M3 &minv, float3 d0, float3 d1, float
     return p > 0.f ? p * length(mul(minv, q_l)) : 0.f;
 }
 
-// Line density of the lobe that was not picked, at the sampled point (out of
-// line: only DR_FLAG_EDGE_LOBE_MIS needs it).
+// The transform into the space of the lobe that was not picked, and its line
+// density at the sampled point (out of line: only DR_FLAG_EDGE_LOBE_MIS needs
+// them).
+DEV M3 other_lobe(const DevScene &s, int mi, const SurfacePoint &sp, float3 wi, const M3 &frame, bool sel_diffuse) {
+    return sel_diffuse ? mul(inverse(ltc_matrix(s, mi, sp, wi)), frame) : frame;
+}
 DEV_NOINLINE float other_lobe_density(const DevScene &s, int mi, const SurfacePoint &sp, float3 wi, const M3 &frame,
                                       bool sel_diffuse, float3 v0, float3 v1, float3 sample_p, float3 q_l) {
-    M3 ominv = sel_diffuse ? mul(inverse(ltc_matrix(s, mi, sp, wi)), frame) : frame;
-    return lobe_line_density(ominv, v0 - sp.p, v1 - sp.p, sample_p, q_l);
+    return lobe_line_density(other_lobe(s, mi, sp, wi, frame, sel_diffuse), v0 - sp.p, v1 - sp.p, sample_p, q_l);
 }
 
-// Secondary edge sample (delta_ray.cpp:45-365), in two phases: the line
-// sample on the edge (edge_line_sample: the silhouette test, the LTC lobe, the
-// point on the edge and the density it was drawn with) and the shading of the
-// two sides (edge_shade_sample: rays, shading, Jacobians).  The backward pass
-// runs them as two kernels with the surviving line samples compacted in
-// between; shading_edge_sample runs both.
+// Secondary edge sample (delta_ray.cpp:45-365), in phases: the line sample on
+// the edge (line_sample_from: the LTC lobe, the point on the edge and the
+// density it was drawn with), the two rays beside it (edge_rays) and the
+// shading of its two sides (edge_shade_hits).  The backward pass runs them as
+// kernels with the surviving samples compacted in between.
 struct EdgeLine {
     float3 sample_p;  // the sampled point on the edge, relative to the shading point
     float3 mwt;       // d sample_p / d l (the lobe transform times the line direction)
@@ -955,81 +977,129 @@ DEV LineSetup line_setup(const DevScene &s, const EdgeSample &es, float3 wi, int
     return ls;
 }
 
-// The line sample of one edge from its point's setup (delta_ray.cpp:88-187):
-// the edge clipped to the lobe's upper hemisphere in LTC space, the point on
-// it drawn by inverting the line integral's CDF (Newton steps guarded by
-// bisection), its density.  EXT adds the lobe mixture weight (sp and wi are
-// read only then).  rec (may be null): the edge's silhouette-test record,
-// which gives the answer of is_silhouette from one contiguous read.
-template <bool EXT = true>
-DEV bool line_sample_from(const DevScene &s, const LineSetup &ls, const EdgeSample &es, const DevEdge &edge, float3 p,
-                          const SurfacePoint &sp, float3 wi, EdgeLine &out, const EdgeRec *rec) {
-    const bool none = false;
-    if (!(rec ? is_silhouette_rec(rec, p) : is_silhouette(s, p, edge))) return none;
-    float3 v0 = edge_v0(s, edge), v1 = edge_v1(s, edge);
-    if (abs_sum(v1 - v0) == 1e-10f) return none;
-    const M3 &minv = ls.minv, &m = ls.m;
-    float3 a = mul(minv, v0 - p), b = mul(minv, v1 - p);
-    if (a.z <= 0.f && b.z <= 0.f) return none;
-    if (a.z < 0.f) a = (a * b.z - b * a.z) / (b.z - a.z);
-    if (b.z < 0.f) b = (a * b.z - b * a.z) / (b.z - a.z);
-    float3 vod = b - a;
-    if (abs_sum(vod) < 1e-10f) return none;
-    float3 wt = normalize(vod);
-    float l0 = dot(a, wt), l1 = dot(b, wt);
-    float3 vo = a - l0 * wt;
-    float d = length(vo);
-    auto I = [&](float l) {
+// The line of one edge in its point's lobe space: vo + l wt at offset l, d its
+// distance from the origin, clipped to the upper hemisphere as [l0, l1]; Il0
+// the line integral's antiderivative at l0 and norm its difference over the
+// range.
+struct LineState {
+    float3 vo, wt;
+    float d, l0, l1, Il0, norm;
+    DEV float integral(float l) const {
         return (l / (d * (d * d + l * l)) + dr_atanf(l / d) / (d * d)) * vo.z + (l * l / (d * (d * d + l * l))) * wt.z;
-    };
-    float Il0 = I(l0), Il1 = I(l1);
-    float norm = Il1 - Il0;
-    if (norm <= 1e-10f) return none;
-    auto cdf = [&](float l) { return (I(l) - Il0) / norm; };
-    auto pdf = [&](float l) {
+    }
+    DEV float pdf(float l) const {
         float ds = d * d + l * l;
         return 2.f * d * (vo + l * wt).z / (norm * ds * ds);
-    };
-    float lb = l0, ub = l1;
-    if (lb > ub) {
-        float t = lb;
-        lb = ub;
-        ub = t;
     }
-    float l = 0.5f * (lb + ub);
-    for (int it = 0; it < 20; it++) {
+};
+// The edge in the lobe's space, clipped to the upper hemisphere as a, b
+// (delta_ray.cpp:107-120); false: it gives no sample.
+DEV bool line_clip(const M3 &minv, float3 v0, float3 v1, float3 p, float3 &a, float3 &b) {
+    if (abs_sum(v1 - v0) == 1e-10f) return false;
+    a = mul(minv, v0 - p);
+    b = mul(minv, v1 - p);
+    if (a.z <= 0.f && b.z <= 0.f) return false;
+    if (a.z < 0.f) a = (a * b.z - b * a.z) / (b.z - a.z);
+    if (b.z < 0.f) b = (a * b.z - b * a.z) / (b.z - a.z);
+    return !(abs_sum(b - a) < 1e-10f);
+}
+// Its line (delta_ray.cpp:121-140); false: it gives no sample.
+DEV bool line_begin(float3 a, float3 b, LineState &ln) {
+    ln.wt = normalize(b - a);
+    ln.l0 = dot(a, ln.wt);
+    ln.l1 = dot(b, ln.wt);
+    ln.vo = a - ln.l0 * ln.wt;
+    ln.d = length(ln.vo);
+    ln.Il0 = ln.integral(ln.l0);
+    ln.norm = ln.integral(ln.l1) - ln.Il0;
+    return !(ln.norm <= 1e-10f);
+}
+
+// The offset l with cdf(l) = u, by up to 20 Newton steps guarded by bisection
+// (delta_ray.cpp:141-160), one step per call; true when l is final.  A short
+// edge's cdf is a difference of nearly equal floats, whose noise keeps the
+// residual above the 1e-5 it is solved to (three in ten samples of a large
+// mesh): the steps then soon repeat a state (l, lb, ub) of the last two, and as
+// a step depends on nothing else, step 19's l is known without taking the rest
+// (9 steps on average instead of 20).
+struct LineSolve {
+    float l, lb, ub;
+    float pl[2], plb[2], pub[2];  // the last two states
+    int it;
+    DEV void begin(const LineState &ln) {
+        lb = ln.l0;
+        ub = ln.l1;
+        if (lb > ub) {
+            float t = lb;
+            lb = ub;
+            ub = t;
+        }
+        l = 0.5f * (lb + ub);
+        it = 0;
+        pl[0] = plb[0] = pub[0] = pl[1] = plb[1] = pub[1] = 0.f;
+    }
+    DEV bool is_state(int k) const {
+        return dr_f2i(l) == dr_f2i(pl[k]) && dr_f2i(lb) == dr_f2i(plb[k]) && dr_f2i(ub) == dr_f2i(pub[k]);
+    }
+    DEV bool step(const LineState &ln, float u) {
         if (!(l >= lb && l <= ub)) l = 0.5f * (lb + ub);
-        float value = cdf(l) - es.u;
-        if (fabsf(value) < 1e-5f || it == 19) break;
+        if (it == 19 || (it > 0 && is_state(0))) return true;
+        if (it > 1 && is_state(1)) {  // the states alternate
+            if ((19 - it) & 1) l = pl[0];
+            return true;
+        }
+        pl[1] = pl[0], plb[1] = plb[0], pub[1] = pub[0];
+        pl[0] = l, plb[0] = lb, pub[0] = ub;
+        float value = (ln.integral(l) - ln.Il0) / ln.norm - u;
+        if (fabsf(value) < 1e-5f) return true;
         if (value > 0.f) ub = l;
         else lb = l;
-        l -= value / pdf(l);
+        l -= value / ln.pdf(l);
+        it++;
+        return false;
     }
-    if (pdf(l) <= 0.f) return none;
-    float3 sample_p = mul(m, vo + l * wt);
+};
+
+// The line sample of one edge from its point's setup (delta_ray.cpp:88-187):
+// the edge clipped to the lobe's upper hemisphere in LTC space, the point on
+// it drawn by inverting the line integral's CDF, its density.  EXT adds the
+// lobe mixture weight (sp and wi are read only then).  The edge is one its
+// point's traversal sampled, so it passed the silhouette test.
+template <bool EXT = true>
+DEV bool line_sample_from(const DevScene &s, const LineSetup &ls, const EdgeSample &es, float3 v0, float3 v1, float3 p,
+                          const SurfacePoint &sp, float3 wi, EdgeLine &out) {
+    LineState ln;
+    float3 a, b;
+    if (!line_clip(ls.minv, v0, v1, p, a, b) || !line_begin(a, b, ln)) return false;
+    LineSolve sv;
+    sv.begin(ln);
+    while (!sv.step(ln, es.u)) {
+    }
+    const float l = sv.l, pdf = ln.pdf(l);
+    if (pdf <= 0.f) return false;
+    float3 sample_p = mul(ls.m, ln.vo + l * ln.wt), mwt = mul(ls.m, ln.wt);
     // DR_FLAG_EDGE_LOBE_MIS: the one-sample balance heuristic over the two
     // lobes, pmf_sel pdf_sel(l) + pmf_other pdf_other(l); the reference divides
     // by pmf_sel pdf_sel(l) alone
-    float q_mix = ls.mpmf * pdf(l);
+    float q_mix = ls.mpmf * pdf;
     if (EXT && s.edge_lobe_mis) {
         bool sel_diffuse = es.bsdf_component <= ls.dpmf;
         float opmf = sel_diffuse ? ls.spmf : ls.dpmf;
         if (opmf > 0.f)
-            q_mix += opmf * other_lobe_density(s, ls.mi, sp, wi, ls.frame, sel_diffuse, v0, v1, sample_p, mul(m, wt));
+            q_mix += opmf * other_lobe_density(s, ls.mi, sp, wi, ls.frame, sel_diffuse, v0, v1, sample_p, mwt);
     }
     out.sample_p = sample_p;
-    out.mwt = mul(m, wt);
+    out.mwt = mwt;
     out.q = q_mix;
     return true;
 }
 
-// rec (may be null): the edge's silhouette-test record.
 template <bool EXT = true>
-DEV bool edge_line_sample(const DevScene &s, const EdgeSample &es, const DevEdge &edge, float3 wi, int stri,
-                          const SurfacePoint &sp, EdgeLine &out, const EdgeRec *rec = nullptr) {
+DEV bool edge_line_sample(const DevScene &s, const EdgeSample &es, const EdgeRec *rec, float3 wi, int stri,
+                          const SurfacePoint &sp, EdgeLine &out) {
     const LineSetup ls = line_setup(s, es, wi, stri, sp);
     if (!ls.ok) return false;
-    return line_sample_from<EXT>(s, ls, es, edge, sp.p, sp, wi, out, rec);
+    return line_sample_from<EXT>(s, ls, es, rec_v0(rec), rec_v1(rec), sp.p, sp, wi, out);
 }
 
 // The two rays of an edge sample, one on each side of the edge: their closest
@@ -1054,26 +1124,21 @@ DEV void edge_side_dirs(const EdgeLine &el, float3 v0, float3 v1, float3 p, floa
 // the operands the LBVH's leaves hold (vertices in index order), for both
 // sides' rays, which share their origin: each face's edge vectors and origin
 // offset serve both rays.
-DEV void hit_faces_pair(const DevScene &s, const DevEdge &edge, float3 o, float3 dr, float3 dl, float tnear, Hit &hr,
-                        Hit &hl) {
-    const int off = s.shapes[edge.shape].tri_off;
-    const int g0 = off + edge.f0, g1 = edge.f1 >= 0 ? off + edge.f1 : -1;
+DEV float4 face_corner(int code, float4 v0, float4 v1, float4 opp) {
+    return code == 0 ? v0 : (code == 1 ? v1 : opp);
+}
+DEV void hit_faces_pair(const EdgeRec *rec, float3 o, float3 dr, float3 dl, float tnear, Hit &hr, Hit &hl) {
+    const float4 v0 = dr_ldg(&rec->r[0]), v1 = dr_ldg(&rec->r[1]), a = dr_ldg(&rec->r[2]), b = dr_ldg(&rec->r[3]);
+    const int corners = dr_f2i(dr_ldg(&rec->r[4].w));
+    const float4 q5 = dr_ldg(&rec->r[5]);
     hr.tri = hl.tri = -1;
     hr.t = hl.t = DR_INF;
-#pragma unroll 1
     for (int k = 0; k < 2; k++) {
-        const int g = k ? g1 : g0;
+        const int g = dr_f2i(k ? q5.y : q5.x), c = corners >> (6 * k);
         if (g < 0) continue;
-        const int4 id = s.tri[g];
-        float4 v[3];
-        const int vi[3] = {id.x, id.y, id.z};
-        for (int j = 0; j < 3; j++) {
-            v[j].x = s.vtx[3 * vi[j]];
-            v[j].y = s.vtx[3 * vi[j] + 1];
-            v[j].z = s.vtx[3 * vi[j] + 2];
-            v[j].w = 0.f;
-        }
-        const TriRay r = tri_ray(v[0], v[1], v[2], o);
+        const float4 opp = k ? b : a;
+        const TriRay r = tri_ray(face_corner(c & 3, v0, v1, opp), face_corner((c >> 2) & 3, v0, v1, opp),
+                                 face_corner((c >> 4) & 3, v0, v1, opp), o);
         float t;
         if (hit_triangle(r, dr, t) && t > tnear && (t < hr.t || (t == hr.t && g < hr.tri))) {
             hr.t = t;
@@ -1086,16 +1151,48 @@ DEV void hit_faces_pair(const DevScene &s, const DevEdge &edge, float3 o, float3
     }
 }
 
+// Whether the two side rays of every sample of the edge surely miss both of
+// its faces, decided before the sample is drawn: the rays lean out of the
+// plane through p and the edge by delta = 1e-3 |sample_p| (edge_side_dirs), so
+// a face must reach that far out of the plane to be hit, and small faces far
+// away do not.  With n the plane's unit normal, X a hit and D the faces' least
+// distance from p, |X . n| >= D (delta - eta) / (1 + delta), eta the angle by
+// which the sample's direction itself may leave the plane (rounding of the
+// lobe's transform m: 1e-6 |m| |x| for points x of the line), while no point
+// of a face has a larger |X . n| than its corner opposite the edge.  Answers
+// true only with a tenth to spare, and 1e-6 |a|^3 / |(v0 - p) x (v1 - p)| for
+// the rounding of n: the hit test's own error is far smaller there (its
+// coordinate of the opposite corner has a relative error of a few
+// 2^-24 / delta, delta - eta being at least 1e-5).
+// L: a bound on the lengths of the line's points x in the lobe's space.
+DEV bool faces_out_of_reach(const EdgeRec *rec, float3 v0, float3 v1, float3 p, const M3 &m, float L) {
+    const float4 qa = dr_ldg(&rec->r[2]), qb = dr_ldg(&rec->r[3]);
+    const float3 d0 = v0 - p, d1 = v1 - p, c = cross(d0, d1);
+    const float l0 = length(d0), len = length(v1 - v0), area = length(c), near = l0 - len;
+    float mm = 0.f;
+    for (int i = 0; i < 9; i++) mm = fmaxf(mm, fabsf(m.m[i]));
+    const float eta = 3e-6f * mm * L / near;  // 3 max |m_ij| bounds |m|
+    const float lean = 1e-3f * near - eta;
+    bool out = near > 0.f && lean > 1e-5f;
+    for (int k = 0; k < 2; k++) {
+        const float4 q = k ? qb : qa;
+        const float3 a = f3(q.x, q.y, q.z) - p;  // v0 or v1 itself where there is no such face
+        const float la = length(a), h = fabsf(dot(a, c)) / area;
+        const float D = l0 - fmaxf(len, length(a - d0));
+        out = out && h + 1e-6f * la * la * la / area < 0.9f * D * lean;
+    }
+    return out;
+}
 
 // The connectivity test of an edge sample in an LBVH scene (most samples
 // end here: edges hidden from p).  A side's closest hit is one of the edge's
 // faces only if its ray hits one of them, at (ta, ida) by the closest-hit
 // rule, and no triangle hits ahead of that.  True if exactly one side is
 // connected: `side` (0 the right ray, 1 the left) and `face`, its closest hit.
-DEV bool edge_connect_bvh(const DevScene &s, const DevEdge &edge, float3 p, float3 rdir, float3 ldir, int &side,
+DEV bool edge_connect_bvh(const DevScene &s, const EdgeRec *rec, float3 p, float3 rdir, float3 ldir, int &side,
                           int &face) {
     Hit fr, fl;
-    hit_faces_pair(s, edge, p, rdir, ldir, 1e-3f, fr, fl);
+    hit_faces_pair(rec, p, rdir, ldir, 1e-3f, fr, fl);
     if (fr.tri < 0 && fl.tri < 0) return false;
     const bool cr = fr.tri >= 0 && !trace_before(s, p, rdir, 1e-3f, fr.t, fr.tri);
     if (!cr && fl.tri < 0) return false;
@@ -1139,13 +1236,13 @@ DEV bool edge_rays_rest(const DevScene &s, int stri, float3 p, float3 rdir, floa
     return true;
 }
 
-DEV bool edge_rays(const DevScene &s, const EdgeLine &el, const DevEdge &edge, int stri, float3 p, bool direct_only,
-                   EdgeHits &out) {
+DEV bool edge_rays(const DevScene &s, const EdgeLine &el, const DevEdge &edge, const EdgeRec *rec, int stri, float3 p,
+                   bool direct_only, EdgeHits &out) {
     float3 sdir, rdir, ldir;
     edge_side_dirs(el, edge_v0(s, edge), edge_v1(s, edge), p, sdir, rdir, ldir);
     if (s.num_tris > DR_LINEAR_TRIS) {
         int side, face;
-        if (!edge_connect_bvh(s, edge, p, rdir, ldir, side, face)) return false;
+        if (!edge_connect_bvh(s, rec, p, rdir, ldir, side, face)) return false;
         return edge_rays_rest(s, stri, p, rdir, ldir, side, face, direct_only, out);
     }
     int hit[2];
@@ -1283,29 +1380,16 @@ DEV EdgeResult edge_shade_hits(const DevScene &s, const EdgeLine &el_, const Dev
 
 // The whole shading of an edge sample: edge_rays, then edge_shade_hits.
 template <bool MAYBE_GI = true>
-DEV EdgeResult edge_shade_sample(const DevScene &s, const EdgeLine &el, const DevEdge &edge, const LightSample &ls,
-                                 const Rng &rng, int nbounces, float3 wi, int stri, const SurfacePoint &sp,
+DEV EdgeResult edge_shade_sample(const DevScene &s, const EdgeLine &el, const DevEdge &edge, const EdgeRec *rec,
+                                 const LightSample &ls, const Rng &rng, int nbounces, float3 wi, int stri, const SurfacePoint &sp,
                                  float3 weight, float3 d_color, bool direct_only) {
     EdgeHits hits;
-    if (!edge_rays(s, el, edge, stri, sp.p, direct_only || !MAYBE_GI, hits)) {
+    if (!edge_rays(s, el, edge, rec, stri, sp.p, direct_only || !MAYBE_GI, hits)) {
         EdgeResult none;
         none.dp = none.dv0 = none.dv1 = f3(0.f);
         return none;
     }
     return edge_shade_hits<MAYBE_GI>(s, el, edge, ls, rng, nbounces, wi, stri, sp, weight, d_color, direct_only, hits);
-}
-
-template <bool EXT = true, bool MAYBE_GI = true>
-DEV EdgeResult shading_edge_sample(const DevScene &s, const EdgeSample &es, const DevEdge &edge, const LightSample &ls,
-                                   const Rng &rng, int nbounces, float3 wi, int stri, const SurfacePoint &sp,
-                                   float3 weight, float3 d_color, bool direct_only) {
-    EdgeLine el;
-    if (!edge_line_sample<EXT>(s, es, edge, wi, stri, sp, el)) {
-        EdgeResult none;
-        none.dp = none.dv0 = none.dv1 = f3(0.f);
-        return none;
-    }
-    return edge_shade_sample<MAYBE_GI>(s, el, edge, ls, rng, nbounces, wi, stri, sp, weight, d_color, direct_only);
 }
 
 // ---------------------------------------------------------------------------

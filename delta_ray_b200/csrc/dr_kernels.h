@@ -176,7 +176,7 @@ struct BackwardWorkspace {
     void *packets;
     long long cap_packets;
     // [cap_points][DR_LCTX_F4] each point's line-sample setup (k_line_ctx;
-    // null: k_edge_line sets it up per edge)
+    // null: k_edge_line_point sets it up per edge)
     float4 *line_ctx;
     // per view of a batched multi-view call (null: the call's own settings);
     // each point's settings are views[point.view]
@@ -222,7 +222,9 @@ cudaError_t dr_launch_edge_traverse(const DevScene &s, uint64_t seed, const Back
 // The silhouette-test records of n tree edges (dr_edges.cuh: edge_record).
 cudaError_t dr_launch_edge_records(const DevScene &s, const DevEdge *edges, int n, EdgeRec *out, cudaStream_t st);
 // Each interior node's children side by side (dr_edges.cuh: pack_children).
-cudaError_t dr_launch_edge_children(const DevEdgeNode *nodes, int n, float4 *box, float4 *dir, cudaStream_t st);
+// recs: the tree's edge records.
+cudaError_t dr_launch_edge_children(const DevEdgeNode *nodes, const EdgeRec *recs, int n, float4 *box, float4 *dir,
+                                    cudaStream_t st);
 // out[b] = edges sampled by points [b P / nb, (b + 1) P / nb) (ws.pt_items)
 cudaError_t dr_launch_item_buckets(const int *pt_items, long long P, int nb, unsigned long long *out,
                                    cudaStream_t st);
@@ -246,7 +248,7 @@ cudaError_t dr_launch_backward_back(const DevScene &s, int W, int H, int spp, in
 // float4 of one point's walk context in BackwardWorkspace::walk_ctx.
 #define DR_CTX_F4 11
 // float4 of one point's line-sample setup in BackwardWorkspace::line_ctx.
-#define DR_LCTX_F4 6
+#define DR_LCTX_F4 9
 
 // Words of one packed secondary-point record in BackwardWorkspace::pt.
 #define DR_PT_FLOATS 24

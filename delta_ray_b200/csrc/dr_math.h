@@ -290,31 +290,35 @@ DRM_FN float dr_cosf(float x) { return (float)drm::cos_d((double)x); }
 // these stay in single precision; every operation is an IEEE float operation
 // without contraction, so the bits are still the same on the GPU and the
 // host).  atan a = k pi/32 + atan t, t = (a - c_k) / (1 + a c_k), with c_k
-// the float nearest tan(k pi/32), k picked by 16 comparisons so that
+// the float nearest tan(k pi/32), k picked by 4 comparisons so that
 // |t| <= ~tan(pi/64), the angle atan(c_k) as a head and a tail float, and the
 // series to t^9; a > ~tan(31 pi/64) as pi/2 - atan(1/a).  Within about 2 ulp.
 namespace drm {
-#define DRM_ATANF_C {0.0f, 0.09849140048027039f, 0.1989123672246933f, 0.3033466935157776f, 0.4142135679721832f, \
-                     0.534511148929596f, 0.6681786179542542f, 0.8206787705421448f, 1.0f, 1.218503475189209f, \
-                     1.4966057538986206f, 1.870868444442749f, 2.4142136573791504f, 3.296558141708374f, \
-                     5.027339458465576f, 10.153170585632324f}
-#define DRM_ATANF_AH {0.0f, 0.09817476570606232f, 0.19634954631328583f, 0.29452431201934814f, \
-                      0.39269909262657166f, 0.49087387323379517f, 0.5890486240386963f, 0.6872233748435974f, \
-                      0.7853981852531433f, 0.8835729360580444f, 0.9817476868629456f, 1.0799224376678467f, \
-                      1.1780972480773926f, 1.2762720584869385f, 1.3744467496871948f, 1.4726215600967407f}
-#define DRM_ATANF_AL {0.0f, 1.8693642189759885e-09f, -5.612990516823402e-09f, 8.32819413432162e-09f, \
-                      -6.148726860999432e-09f, -1.1015669265646011e-08f, -1.5293277755290546e-08f, \
-                      6.007060626700422e-09f, -2.1855694143368964e-08f, -2.2519143882959725e-08f, \
-                      1.4677898008130796e-08f, 4.425970701049664e-08f, 1.0932094340887488e-08f, \
-                      -4.863122882170501e-08f, 3.4977222895804516e-08f, -1.8240424726201354e-09f}
+// rows (c_k, head and tail of atan c_k, 0): one 16-byte read per row on the device
+struct alignas(16) AtanRow {
+    float c, ah, al, pad;
+};
+#define DRM_ATANF_ROWS { \
+    {0.0f, 0.0f, 0.0f, 0.f}, \
+    {0.09849140048027039f, 0.09817476570606232f, 1.8693642189759885e-09f, 0.f}, \
+    {0.1989123672246933f, 0.19634954631328583f, -5.612990516823402e-09f, 0.f}, \
+    {0.3033466935157776f, 0.29452431201934814f, 8.32819413432162e-09f, 0.f}, \
+    {0.4142135679721832f, 0.39269909262657166f, -6.148726860999432e-09f, 0.f}, \
+    {0.534511148929596f, 0.49087387323379517f, -1.1015669265646011e-08f, 0.f}, \
+    {0.6681786179542542f, 0.5890486240386963f, -1.5293277755290546e-08f, 0.f}, \
+    {0.8206787705421448f, 0.6872233748435974f, 6.007060626700422e-09f, 0.f}, \
+    {1.0f, 0.7853981852531433f, -2.1855694143368964e-08f, 0.f}, \
+    {1.218503475189209f, 0.8835729360580444f, -2.2519143882959725e-08f, 0.f}, \
+    {1.4966057538986206f, 0.9817476868629456f, 1.4677898008130796e-08f, 0.f}, \
+    {1.870868444442749f, 1.0799224376678467f, 4.425970701049664e-08f, 0.f}, \
+    {2.4142136573791504f, 1.1780972480773926f, 1.0932094340887488e-08f, 0.f}, \
+    {3.296558141708374f, 1.2762720584869385f, -4.863122882170501e-08f, 0.f}, \
+    {5.027339458465576f, 1.3744467496871948f, 3.4977222895804516e-08f, 0.f}, \
+    {10.153170585632324f, 1.4726215600967407f, -1.8240424726201354e-09f, 0.f}}
 #if defined(__CUDACC__)
-static __device__ const float drm_atanf_c_dev[16] = DRM_ATANF_C;
-static __device__ const float drm_atanf_ah_dev[16] = DRM_ATANF_AH;
-static __device__ const float drm_atanf_al_dev[16] = DRM_ATANF_AL;
+static __device__ const AtanRow drm_atanf_dev[16] = DRM_ATANF_ROWS;
 #endif
-static const float drm_atanf_c_host[16] = DRM_ATANF_C;
-static const float drm_atanf_ah_host[16] = DRM_ATANF_AH;
-static const float drm_atanf_al_host[16] = DRM_ATANF_AL;
+static const AtanRow drm_atanf_host[16] = DRM_ATANF_ROWS;
 constexpr float kPio2Hf = 1.5707963705062866f, kPio2Lf = -4.371138828673793e-08f;
 constexpr float kPiHf = 3.1415927410125732f, kPiLf = -8.742277657347586e-08f;
 
@@ -360,15 +364,21 @@ DRM_FN float atanf_pos(float a) {
         float t = fdiv(1.f, a);
         return fadd(kPio2Hf, fsub(kPio2Lf, fadd(t, atanf_tail(t))));
     }
-    int k = (a > 0.049126848578453064f) + (a > 0.1483359932899475f) + (a > 0.25048696994781494f) +
-            (a > 0.3578057289123535f) + (a > 0.4729647636413574f) + (a > 0.599376916885376f) +
-            (a > 0.7416505217552185f) + (a > 0.9063471555709839f) + (a > 1.1033300161361694f) +
-            (a > 1.3483439683914185f) + (a > 1.6683992147445679f) + (a > 2.1143224239349365f) +
-            (a > 2.7948126792907715f) + (a > 3.9922237396240234f) + (a > 6.741452217102051f);
+    // k: how many of the 15 thresholds a exceeds, by halving
+    const bool k8 = a > 0.9063471555709839f;
+    const bool k4 = a > (k8 ? 2.1143224239349365f : 0.3578057289123535f);
+    const bool k2 = a > (k8 ? (k4 ? 3.9922237396240234f : 1.3483439683914185f)
+                            : (k4 ? 0.599376916885376f : 0.1483359932899475f));
+    const float last = k8 ? (k4 ? (k2 ? 6.741452217102051f : 2.7948126792907715f)
+                                : (k2 ? 1.6683992147445679f : 1.1033300161361694f))
+                          : (k4 ? (k2 ? 0.7416505217552185f : 0.4729647636413574f)
+                                : (k2 ? 0.25048696994781494f : 0.049126848578453064f));
+    const int k = (k8 ? 8 : 0) + (k4 ? 4 : 0) + (k2 ? 2 : 0) + (a > last ? 1 : 0);
 #ifdef __CUDA_ARCH__
-    float c = __ldg(&drm_atanf_c_dev[k]), ah = __ldg(&drm_atanf_ah_dev[k]), al = __ldg(&drm_atanf_al_dev[k]);
+    const float4 row = __ldg(reinterpret_cast<const float4 *>(drm_atanf_dev) + k);
+    const float c = row.x, ah = row.y, al = row.z;
 #else
-    float c = drm_atanf_c_host[k], ah = drm_atanf_ah_host[k], al = drm_atanf_al_host[k];
+    const float c = drm_atanf_host[k].c, ah = drm_atanf_host[k].ah, al = drm_atanf_host[k].al;
 #endif
     float t = fdiv(fsub(a, c), fadd(1.f, fmul(a, c)));
     return fadd(ah, fadd(al, fadd(t, atanf_tail(t))));

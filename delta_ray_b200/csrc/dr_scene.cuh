@@ -46,13 +46,16 @@ struct DevLight {
 
 struct DevEdge { int shape, v0, v1, f0, f1; };  // local vertex / triangle ids
 
-// What the silhouette test of a tree edge needs, computed once per scene
-// build (dr_edges.cuh: edge_record): its end points v0, v1, the vertices a, b
-// of its two faces opposite it and the faces' unit normals n0, n1;
-// r[0] = (v0, n0.x), r[1] = (v1, n0.y), r[2] = (a, n0.z), r[3] = (b, n1.x),
-// r[4] = (n1.y, n1.z, always, 0): always != 0 for edges that are silhouettes
-// from everywhere (no shading normals, or one face).
-struct EdgeRec { float4 r[5]; };
+// What a tree edge's silhouette test, line sample and face hits need, computed
+// once per scene build (dr_edges.cuh: edge_record): its end points v0, v1, the
+// vertices a, b of its two faces opposite it, the faces' unit normals n0, n1
+// and the faces themselves; r[0] = (v0, n0.x), r[1] = (v1, n0.y), r[2] = (a,
+// n0.z), r[3] = (b, n1.x), r[4] = (n1.y, n1.z, always, corners as int bits),
+// r[5] = (global triangle ids of the faces as int bits, -1 for none; 0, 0).
+// always != 0: edges that are silhouettes from everywhere (no shading normals,
+// or one face; n0 and n1 are 0).  corners: which of v0, v1 and the opposite
+// vertex (0, 1, 2) each corner of face k is, 2 bits each from bit 6 k.
+struct EdgeRec { float4 r[6]; };
 
 struct DevEdgeNode {
     float lo[3], hi[3];
