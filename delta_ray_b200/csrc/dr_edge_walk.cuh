@@ -2,38 +2,48 @@
 // batch of points with its pending nodes in shared memory.  Included by
 // dr_edge_kernels.cu.
 //
-// What bounds it: the node decisions' arithmetic (about 350 instructions per
-// child, most of them the BSDF bound's) and the latency of the node reads
-// between them.  Two lanes share a node, one per child, so that a lane
-// evaluates one bound, reads its child with two 16-byte loads next to its
-// partner's, and exchanges importances and tests with one shuffle each: 16
-// nodes a step.  The nodes come off two stacks by class (class 0 takes the cone tests
-// and the exact bounds, class 1 mostly filtered ones), so that the lanes of a
-// step mostly run one path.  The points' contexts, the stacks, the reached
-// leaves and the sampled edges stay in shared memory: a node costs no global
-// traffic but its own record, and the items leave in runs of consecutive
-// slots, each point's together (the line and ray kernels then read one
-// point's data and neighbouring edges from a warp's lanes).
+// What bounds it: instruction issue and fetch (a node decision is 300 to 450
+// instructions per child, most of them the BSDF bound's).  Two lanes share a
+// node, one per child, so that a lane evaluates one bound, reads its child
+// with two 16-byte loads next to its partner's, and exchanges importances and
+// tests with one shuffle each: 16 nodes a step.  The nodes come off stacks by
+// class, so that the lanes of a step run one path: the nodes that split the all
+// walk (three in four of a glossy heightfield's) need no draw, no cone tests
+// and only a bound's sides of 0 and 1.  The points' contexts, the stacks, the
+// reached leaves and the sampled edges stay in shared memory: a node costs no
+// global traffic but its own record, and the items leave in runs of
+// consecutive slots, each point's together (the line and ray kernels then read
+// one point's data and neighbouring edges from a warp's lanes).
 //
 // Measured against the walk it replaced (one level of every point's nodes
 // per launch, nodes queued in global memory between levels, the point's
 // 176-byte context read per node), level and leaf kernels against this one:
 // the 130,054-triangle heightfield at 640x480, 1 spp (1.16 G nodes): 254 ->
-// 78.6 ms, at 160x120 (72 M): 22.6 -> 5.7; a 64x64-vertex heightfield at
+// 65 ms, at 160x120 (72 M): 22.6 -> 4.6; a 64x64-vertex heightfield at
 // 128x96, 8 spp (53 M): 7.9 -> 5.4; a room of smooth spheres (28 M nodes, 90
-// per point): 6.0 -> 5.1.  25.8 of 32 lanes are active (10 before).  Without
-// the rounds the first took 184 ms and the second 20.7: its few longest walks
-// ran alone.
+// per point): 6.0 -> 5.3.  24 of 32 lanes are active (10 before).  Without
+// the rounds the first took 184 ms and the second 20.7 (its few longest walks
+// ran alone); with one step for every node that splits or draws 83 and 5.9.
 #pragma once
 
-// Pending nodes per warp.  A step takes k <= 16 nodes of one class and adds at
-// most 2 k: it takes only as many as leave DR_WALK_RESERVE slots of its class
-// free, and at least one.  Taking one at a time needs one slot per tree level
-// (trees are split at the median: at most 28 levels, node ids having 27
-// bits), so the reserve always suffices.  A class-0 step also adds up to 32
-// nodes to class 1, of which it finds fewer than 16.
-#define DR_WALK_N1 320
-#define DR_WALK_N0 224
+// Pending nodes per warp, by class: 2 the all walk's nodes that split (bound
+// above 1, or around the point), whose children's bounds only meet thresholds
+// and whose cone tests decide nothing (k_edge_walk's fast step; three in four
+// nodes of a glossy heightfield); of the others, 1 the all walk's off the cone
+// walk's path, 0 the rest, which take the cone tests.
+//
+// While all stacks have room for a step's children the classes are stepped as
+// they fill.  Without that room (or room to hand the nodes on) no node goes to
+// class 2 any more (`two`): a child then stays in its parent's class or goes to
+// class 1, and a step takes only as many nodes as leave
+// DR_WALK_RESERVE slots of its class free, and at least one.  Taking one at a
+// time needs one slot per tree level (trees are split at the median: at most
+// 28 levels, node ids having 27 bits), so the reserve always suffices; steps
+// of classes 0 and 2 also add up to 32 nodes to the classes below, which are
+// drained first.
+#define DR_WALK_N0 128
+#define DR_WALK_N1 128
+#define DR_WALK_N2 224
 #define DR_WALK_RESERVE 32
 #define DR_WALK_POINTS 4  // points of a batch, at most
 #define DR_WALK_ITEMS 128
@@ -109,14 +119,22 @@ struct WalkCtx {
     }
 };
 
+// The exact bound of a box, out of line: the walk's loop must stay within the
+// instruction cache (with this and the silhouette test's exact part inlined
+// where they are needed the fast step ran no faster than the general one,
+// waiting on instruction fetches for half of its cycles).
+static __device__ __noinline__ float walk_bound(float3 lo, float3 hi, const float *ctx) {
+    return bsdf_bound_box(lo, hi, WalkCtx{ctx}.bound(), nullptr);
+}
+
 // One warp's shared memory.  A pending node's code: node id, the point's slot
 // in the batch << 27, mode << 30, all-split << 31.
 template <bool PROP> struct WalkWarp {
     static constexpr int kCtx = PROP ? 44 : 32;  // words of a context
     float4 ctx[DR_WALK_POINTS][kCtx / 4 + 1];    // one float4 of padding: slots start in different banks
-    uint2 s0[DR_WALK_N0], s1[DR_WALK_N1];  // pending nodes by class: code, apmf
-    float c0[DR_WALK_N0];                  // class 0's cpmf (class 1's is 0)
-    float l0[PROP ? DR_WALK_N0 : 1], l1[PROP ? DR_WALK_N1 : 1];  // lpmf
+    uint2 st[DR_WALK_N0 + DR_WALK_N1 + DR_WALK_N2];  // pending nodes, class after class: code, apmf
+    float c[DR_WALK_N0 + DR_WALK_N2];                // cpmf of classes 0 and 2 (class 1's is 0)
+    float l[PROP ? DR_WALK_N0 + DR_WALK_N1 + DR_WALK_N2 : 1];  // lpmf
     uint2 leaf[64];        // edge or node | slot << 27 | mode << 30 | many << 31, weight
     uint2 item[DR_WALK_ITEMS];  // edge | slot << 27 | mode << 30, weight
     uint8_t item_code[PROP ? DR_WALK_ITEMS : 1];
@@ -165,25 +183,32 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
         if (lane < DR_WALK_POINTS) sh.cnt[lane] = 0;
         __syncwarp();
         const auto ctx_of = [&](int slot) { return WalkCtx{reinterpret_cast<const float *>(sh.ctx[slot])}; };
-        int n0 = 0, n1 = 0, nl = 0, ni = 0;  // pending nodes by class, leaves, items
-        if (in) {  // the handed-on nodes, to their classes
+        int n0 = 0, n1 = 0, n2 = 0, nl = 0, ni = 0;  // pending nodes by class, leaves, items
+        bool two = out != nullptr;                   // nodes may go to class 2
+        // a node to its class's stack, every lane's at once
+        const int b1 = DR_WALK_N0, b2 = DR_WALK_N0 + DR_WALK_N1;  // where classes 1 and 2 begin
+        const auto push_nodes = [&](bool node, unsigned code, float cp, float ap, float lp) {
+            const bool all_walk = (code >> 30) & 1;
+            const bool to2 = node && two && all_walk && (code >> 31), to0 = node && !to2 && (!all_walk || cp != 0.f);
+            const unsigned m0 = __ballot_sync(full, to0), m2 = __ballot_sync(full, to2),
+                           m1 = __ballot_sync(full, node && !to0 && !to2);
+            if (node) {
+                const int at = to0 ? n0 + __popc(m0 & below)
+                                   : (to2 ? b2 + n2 + __popc(m2 & below) : b1 + n1 + __popc(m1 & below));
+                sh.st[at] = make_uint2(code, __float_as_uint(ap));
+                if (to0) sh.c[at] = cp;
+                else if (to2) sh.c[at - DR_WALK_N1] = cp;
+                if constexpr (PROP) sh.l[at] = lp;
+            }
+            n0 += __popc(m0);
+            n1 += __popc(m1);
+            n2 += __popc(m2);
+        };
+        if (in) {  // the handed-on nodes
             const bool have = lane < pk->count;
             uint4 e = make_uint4(0, 0, 0, 0);
             if (have) e = pk->e[lane];
-            const bool c0 = have && (!((e.x >> 30) & 1) || __uint_as_float(e.z) != 0.f);
-            const unsigned m0 = __ballot_sync(full, c0), m1 = __ballot_sync(full, have && !c0);
-            if (c0) {
-                const int at = __popc(m0 & below);
-                sh.s0[at] = make_uint2(e.x, e.y);
-                sh.c0[at] = __uint_as_float(e.z);
-                if constexpr (PROP) sh.l0[at] = __uint_as_float(e.w);
-            } else if (have) {
-                const int at = __popc(m1 & below);
-                sh.s1[at] = make_uint2(e.x, e.y);
-                if constexpr (PROP) sh.l1[at] = __uint_as_float(e.w);
-            }
-            n0 = __popc(m0);
-            n1 = __popc(m1);
+            push_nodes(have, e.x, __uint_as_float(e.z), __uint_as_float(e.y), __uint_as_float(e.w));
             __syncwarp();
         } else {  // both walks of every point start at the root of its tree
             bool valid = false, leaf = false;
@@ -199,10 +224,10 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
             const unsigned mask = __ballot_sync(full, valid && !leaf), ml = __ballot_sync(full, leaf);
             if (valid && !leaf) {
                 const int at = 2 * __popc(mask & below);
-                sh.s0[at] = make_uint2(code, __float_as_uint(pmf));
-                sh.s0[at + 1] = make_uint2(code | (1u << 30), __float_as_uint(pmf));
-                sh.c0[at] = sh.c0[at + 1] = pmf;
-                if constexpr (PROP) sh.l0[at] = sh.l0[at + 1] = pmf;
+                sh.st[at] = make_uint2(code, __float_as_uint(pmf));
+                sh.st[at + 1] = make_uint2(code | (1u << 30), __float_as_uint(pmf));
+                sh.c[at] = sh.c[at + 1] = pmf;
+                if constexpr (PROP) sh.l[at] = sh.l[at + 1] = pmf;
             } else if (leaf) {  // a tree of one node: both walks reach it
                 float a = pmf;
                 if constexpr (PROP) a = ws.proposal_alpha * pmf + (1.f - ws.proposal_alpha) * pmf;
@@ -287,11 +312,13 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
                 if (ni > DR_WALK_ITEMS - 32) flush();
             }
         };
-        for (int steps = 0; n0 + n1 > 0; steps++) {
-            if (out && steps >= DR_WALK_STEPS && n0 + n1 >= DR_WALK_HAND) {
+        for (int steps = 0; n0 + n1 + n2 > 0; steps++) {
+            const bool room = n0 <= DR_WALK_N0 - DR_WALK_RESERVE - 32 && n1 <= DR_WALK_N1 - DR_WALK_RESERVE - 32 &&
+                              n2 <= DR_WALK_N2 - 32;
+            if (two && (!room || (steps >= DR_WALK_STEPS && n0 + n1 + n2 >= DR_WALK_HAND))) {
                 // the pending nodes to the next round: packet q of np takes
                 // every np-th, so that large and small subtrees spread
-                const int n = n0 + n1, np = (n + 31) >> 5;
+                const int n = n0 + n1 + n2, np = (n + 31) >> 5;
                 unsigned long long first = 0;
                 if (lane == 0) first = atomicAdd(&ws.counters->walk_n[round], (unsigned long long)np);
                 first = __shfl_sync(full, first, 0);
@@ -301,12 +328,12 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
                     WalkPacket *o = out + first + q;
                     const int i = q + lane * np;
                     if (fits && i < n) {
-                        const bool c0 = i < n0;
-                        const int at = c0 ? i : i - n0;
-                        const uint2 e = c0 ? sh.s0[at] : sh.s1[at];
+                        const int at = i < n0 ? i : (i < n0 + n1 ? b1 + i - n0 : b2 + i - n0 - n1);
+                        const uint2 e = sh.st[at];
                         float l = 0.f;
-                        if constexpr (PROP) l = c0 ? sh.l0[at] : sh.l1[at];
-                        o->e[lane] = make_uint4(e.x, e.y, c0 ? __float_as_uint(sh.c0[at]) : 0u, __float_as_uint(l));
+                        if constexpr (PROP) l = sh.l[at];
+                        const float cp = at < b1 ? sh.c[at] : (at >= b2 ? sh.c[at - DR_WALK_N1] : 0.f);
+                        o->e[lane] = make_uint4(e.x, e.y, __float_as_uint(cp), __float_as_uint(l));
                     }
                     // no room for all: the packets there is room for are left
                     // empty and the warp walks on itself
@@ -316,29 +343,47 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
                     }
                     if (fits && lane < nb) o->point[lane] = sh.point[lane];
                 }
-                steps = -(1 << 30);
                 if (fits) break;
+                two = false;
             }
-            // take up to 16 nodes of one class: class 1 while a step of it is
-            // full (its children stay in class 1, so its stack drains), class
-            // 0 otherwise, and the rest of class 1 last
-            const bool cls0 = n1 < 16 && n0 > 0;
-            const int k = cls0 ? min(min(16, n0), max(1, DR_WALK_N0 - n0 - DR_WALK_RESERVE))
-                               : min(min(16, n1), max(1, DR_WALK_N1 - n1 - DR_WALK_RESERVE));
+            // Up to 16 nodes: of one class where a class fills the step, else of
+            // all (which only the general step takes).  k0, k1, k2: the nodes
+            // taken of each class.
+            int k0 = 0, k1 = 0, k2 = 0;
+            const bool fast = two && n2 >= 16;
+            if (fast) {
+                k2 = 16;
+            } else if (!two) {  // short of room: class 1 first, then 0, which add to none but themselves and 1
+                if (n1 >= 16) k1 = min(16, max(1, DR_WALK_N1 - n1 - DR_WALK_RESERVE));
+                else if (n0 >= 16) k0 = min(16, max(1, DR_WALK_N0 - n0 - DR_WALK_RESERVE));
+                else if (n2 > 0) k2 = min(16, n2);
+                else if (n0 > 0) k0 = min(min(16, n0), max(1, DR_WALK_N0 - n0 - DR_WALK_RESERVE));
+                else k1 = n1;
+            } else if (n1 >= 16) {
+                k1 = 16;
+            } else if (n0 >= 16) {
+                k0 = 16;
+            } else {
+                k2 = n2;
+                k1 = min(n1, 16 - k2);
+                k0 = min(n0, 16 - k2 - k1);
+            }
+            const int k = k0 + k1 + k2;
             const int j = lane >> 1;
             const bool right = lane & 1, act = j < k;
             unsigned code = 0;
             float cpmf = 0.f, apmf = 0.f, lpmf = 0.f;
             if (act) {
-                const int at = (cls0 ? n0 : n1) - 1 - j;
-                const uint2 e = cls0 ? sh.s0[at] : sh.s1[at];
+                const int at = j < k2 ? b2 + n2 - 1 - j : (j < k2 + k1 ? b1 + n1 - 1 - (j - k2) : n0 - 1 - (j - k2 - k1));
+                const uint2 e = sh.st[at];
                 code = e.x;
                 apmf = __uint_as_float(e.y);
-                if (cls0) cpmf = sh.c0[at];
-                if constexpr (PROP) lpmf = cls0 ? sh.l0[at] : sh.l1[at];
+                cpmf = at < b1 ? sh.c[at] : (at >= b2 ? sh.c[at - DR_WALK_N1] : 0.f);
+                if constexpr (PROP) lpmf = sh.l[at];
             }
-            if (cls0) n0 -= k;
-            else n1 -= k;
+            n0 -= k0;
+            n1 -= k1;
+            n2 -= k2;
             visits += k;
             __syncwarp();
             const int nid = (int)(code & DR_NODE_MASK), slot = (code >> 27) & 7;
@@ -365,29 +410,47 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
                     cs = cone_reaches_silhouette(sphere_center(lo, hi), d1.x, f3(d0.x, d0.y, d0.z), d0.w, d1.y, d1.z, p);
                 }
             }
+            // what becomes of the child: walked, its share of the walks
+            bool push = false;
+            float bb = 0.f, ccpmf = cpmf, capmf = apmf, clpmf = lpmf;
+            if (fast) {
+                // a node that splits: a child is walked if it can hold a
+                // silhouette and its bound is above 0, as long as the two
+                // importances are above the cutoff; its shares of both walks
+                // are the node's
+                float fm = 0.f, imp = 0.f;
+                if (cs) {
+                    if (!bsdf_bound_side(lo, hi, cx.bound(), bb, fm)) bb = walk_bound(lo, hi, cx.w);
+                    imp = filt_div(bb * len, length_sq(p - 0.5f * (lo + hi)));
+                }
+                float sum = imp + __shfl_xor_sync(full, imp, 1);
+                fm = fmaxf(fm, __shfl_xor_sync(full, fm, 1));
+                const bool open = !(sum > 1e-10f * (1.0001f + 2.f * fm) || sum < 1e-10f * (0.9999f - 2.f * fm));
+                if (__any_sync(full, act && open)) {
+                    if (open && cs) {
+                        bb = walk_bound(lo, hi, cx.w);
+                        imp = box_importance(lo, hi, len, bb, p);
+                    }
+                    const float exact = imp + __shfl_xor_sync(full, imp, 1);
+                    if (open) sum = exact;
+                }
+                push = cs && !(sum <= 1e-10f) && !(bb <= 0.f);
+            } else {
             // its bound and importance (node_children's rules)
-            const bool filt = !cone_mode && all_split && cpmf == 0.f;
-            float fm = 0.f, bb = 0.f, imp = 0.f;
+            float imp = 0.f;
             if (cs) {
-                bb = bsdf_bound_box(lo, hi, cx.bound(), filt ? &fm : nullptr);
+                bb = walk_bound(lo, hi, cx.w);
                 imp = box_importance(lo, hi, len, bb, p);
             }
-            float oimp = __shfl_xor_sync(full, imp, 1);
-            const float ofm = __shfl_xor_sync(full, fm, 1);
-            const bool open = (fm > 0.f || ofm > 0.f) &&
-                              filter_undecided(right ? oimp : imp, right ? imp : oimp, right ? ofm : fm, right ? fm : ofm);
-            if (__any_sync(full, open)) {
-                if (open && cs) {
-                    bb = bsdf_bound_box(lo, hi, cx.bound(), nullptr);
-                    imp = box_importance(lo, hi, len, bb, p);
-                }
-                oimp = __shfl_xor_sync(full, imp, 1);
-            }
+            const float oimp = __shfl_xor_sync(full, imp, 1);
             const bool ocs = __shfl_xor_sync(full, (int)cs, 1);
             const float il = right ? oimp : imp, ir = right ? imp : oimp;
             bool walk = act && !(il + ir <= 1e-10f);
             bool hc = false;
-            const bool cone_tests = walk && (cone_mode || cpmf != 0.f || !dr_isfinite(il) || !dr_isfinite(ir));
+            // (a node that splits the all walk gives each child its whole share
+            // whatever the cone tests say)
+            const bool cone_tests =
+                walk && (cone_mode || (!all_split && (cpmf != 0.f || !dr_isfinite(il) || !dr_isfinite(ir))));
             if (__any_sync(full, cone_tests)) {
                 if (cone_tests) hc = box_cone_box(lo, hi, cx.cone());
             }
@@ -410,7 +473,6 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
                     pl = right ? 1.f - plleft : plleft;
                 }
             }
-            bool push = false;
             if (walk) {
                 if (cone_mode ? sh2.cone_split : all_split) {
                     push = cs && !(bb <= 0.f);
@@ -420,8 +482,10 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
                     push = ((u < pick) != right) && !(bb <= 0.f);
                 }
             }
-            const float ccpmf = (right ? sh2.prc : sh2.plc) * cpmf, capmf = (right ? sh2.pra : sh2.pla) * apmf;
-            const float clpmf = pl * lpmf;
+            ccpmf = (right ? sh2.prc : sh2.plc) * cpmf;
+            capmf = (right ? sh2.pra : sh2.pla) * apmf;
+            clpmf = pl * lpmf;
+            }
             const bool leaf = push && (child & DR_CHILD_LEAF);
             float w = 0.f;
             if (leaf) {  // EdgeWalk::leaf's weight; no item of weight 0 is kept
@@ -434,24 +498,12 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
             // the others wait for their test
             const bool sure = leaf && w != 0.f && (child & DR_CHILD_SURE) && !(PROP && ws.train_targets);
             const bool keep = leaf && w != 0.f && !sure, node = push && !leaf;
-            const bool to0 = node && (cone_mode || ccpmf != 0.f), to1 = node && !to0;
-            const unsigned m0 = __ballot_sync(full, to0), m1 = __ballot_sync(full, to1),
-                           ml = __ballot_sync(full, keep), ms = __ballot_sync(full, sure);
+            const unsigned ml = __ballot_sync(full, keep), ms = __ballot_sync(full, sure);
             visits += __popc(__ballot_sync(full, leaf));
             const unsigned tag = code & (15u << 27);  // slot and mode
-            if (node) {
-                const unsigned cc = tag | (unsigned)child | ((bb > 1.f || box_inside(lo, hi, p)) ? 1u << 31 : 0u);
-                if (to0) {
-                    const int at = n0 + __popc(m0 & below);
-                    sh.s0[at] = make_uint2(cc, __float_as_uint(capmf));
-                    sh.c0[at] = ccpmf;
-                    if constexpr (PROP) sh.l0[at] = clpmf;
-                } else {
-                    const int at = n1 + __popc(m1 & below);
-                    sh.s1[at] = make_uint2(cc, __float_as_uint(capmf));
-                    if constexpr (PROP) sh.l1[at] = clpmf;
-                }
-            } else if (keep) {
+            push_nodes(node, tag | (unsigned)child | ((bb > 1.f || box_inside(lo, hi, p)) ? 1u << 31 : 0u), ccpmf, capmf,
+                       clpmf);
+            if (keep) {
                 sh.leaf[nl + __popc(ml & below)] =
                     make_uint2(tag | (unsigned)(child & DR_NODE_MASK) | ((child & DR_CHILD_MANY) ? 1u << 31 : 0u),
                                __float_as_uint(w));
@@ -463,8 +515,6 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, B
             }
             if (nb == 1 && lane == 0) sh.cnt[0] += __popc(ms);
             ni += __popc(ms);
-            n0 += __popc(m0);
-            n1 += __popc(m1);
             nl += __popc(ml);
             __syncwarp();
             if (ni > DR_WALK_ITEMS - 32) flush();

@@ -251,6 +251,12 @@ DEV float filt_rsqrt(float x) { return rsqrtf(x); }
 DEV float filt_log2(float x) { return log2f(x); }
 DEV float filt_exp2(float x) { return exp2f(x); }
 #endif
+// a / b to a few ulps (b > 0 and not huge)
+#ifdef DR_HOST_BUILD
+HD float filt_div(float a, float b) { return a / b; }
+#else
+DEV float filt_div(float a, float b) { return __fdividef(a, b); }
+#endif
 
 // The largest and the smallest of dot(d, corner - p) over a box's corners,
 // q: lo - p, hi - p per axis (x0 x1 y0 y1 z0 z1).  Each corner's dot is
@@ -333,6 +339,57 @@ DEV float bsdf_bound_box(float3 blo, float3 bhi, const BoundCtx &c, float *fast_
     return cos_max * (c.dl / DR_PI + c.sl * maxp);
 }
 
+// A Blinn-Phong bound known only by its sides of 0 and 1, for nodes whose
+// children's bounds meet nothing else: as the filtered form of bsdf_bound_box,
+// but with fast divisions and square roots, whose errors of a few ulps widen
+// the margin.  hdn, the largest cosine between the normal and a half vector,
+// has an error of at most 4e-6 (1 + 1 / shmax) (its sine comes from 1 -
+// chmax^2, whose root passes on an error of 1e-6 as 1e-6 / shmax).  False
+// where a step divides by or roots something too near 0 for that, where the
+// margin is wide and where the bound is within it of 1: the exact bound is
+// needed then.  fm: the bound's relative margin.
+DEV bool bsdf_bound_side(float3 blo, float3 bhi, const BoundCtx &c, float &bound, float &fm) {
+    bound = fm = 0.f;
+    if (c.sl > 0.f && c.model != DR_MICROFACET_GGX) {
+        const float q[6] = {blo.x - c.p.x, bhi.x - c.p.x, blo.y - c.p.y, bhi.y - c.p.y, blo.z - c.p.z, bhi.z - c.p.z};
+        if (!(corner_range(c.n, q).hi > 0.f)) return true;
+        const DotRange rx = corner_range(c.hf.t, q), ry = corner_range(c.hf.b, q), rz = corner_range(c.hf.n, q);
+        const float3 lo = f3(rx.lo, ry.lo, rz.lo), hi = f3(rx.hi, ry.hi, rz.hi);
+        const float hx = hi.x;
+        const float cphi = hx * filt_rsqrt((hx > 0.f ? min_sq_bound(lo.y, hi.y) : max_sq_bound(lo.y, hi.y)) + hx * hx);
+        const float dmin = lo.z > 0.f ? max_sq_bound(lo.x, hi.x) + max_sq_bound(lo.y, hi.y)
+                                      : min_sq_bound(lo.x, hi.x) + min_sq_bound(lo.y, hi.y);
+        const float dmax = hi.z > 0.f ? min_sq_bound(lo.x, hi.x) + min_sq_bound(lo.y, hi.y)
+                                      : max_sq_bound(lo.x, hi.x) + max_sq_bound(lo.y, hi.y);
+        const float tmin = (filt_div(lo.z, dmin + lo.z * lo.z) + 1.f) / 2.f,
+                    tmax = (filt_div(hi.z, dmax + hi.z * hi.z) + 1.f) / 2.f;
+        const float3 ln = c.ln;
+        const float u = ln.x * cphi, zz = ln.z * ln.z;
+        const float cth_min = tmin * filt_rsqrt(tmin), cth_max = tmax * filt_rsqrt(tmax);
+        const float ch0 = cphi >= 0.f ? fabsf(ln.z) * filt_rsqrt(zz + u * u) : 1.f;
+        const float ch = ch0 > cth_max ? cth_max : (ch0 < cth_min ? cth_min : ch0);
+        // the sine; exactly 0 for the constant cosine 1, and above a cosine of 1
+        const bool one = !(cphi >= 0.f) && ch == 1.f;
+        const float s2 = 1.f - ch * ch, rs = s2 > 0.f ? filt_rsqrt(s2) : 0.f, sh = s2 * rs;
+        const float hdn = fminf(fabsf(u * sh) + ln.z * ch, 1.f);
+        const float e = c.expo, y = e * filt_log2(hdn);
+        // tmin, tmax and s2 clear of 0 (a negative tmin or tmax gives NaN here as
+        // in the exact evaluation, and clamps nothing), and ch0 clear of
+        // cth_max, where the clamp jumps if cth_min is larger
+        const bool sound = fabsf(tmin) > 1e-3f && fabsf(tmax) > 1e-3f && fabsf(tmin) < 100.f && fabsf(tmax) < 100.f &&
+                           (one || fabsf(s2) > 1e-4f) && hdn > 1e-2f && fabsf(hx) > 1e-15f &&
+                           !(fabsf(ch0 - cth_max) < 2e-5f);
+        const float m = (16.f + fabsf(y)) * 2.384185791e-7f + e * filt_div(8e-6f * (1.f + rs), hdn);
+        const float bf = c.dl / DR_PI + c.sl * (filt_exp2(y) * (e + 2.f) / float(2 * 3.14159265358979323846));
+        if (sound && y > -120.f && m < 0.01f && bf > 1e-30f && (bf * (1.f - m) > 1.f || bf * (1.f + m) <= 1.f)) {
+            bound = bf;
+            fm = m;
+            return true;
+        }
+    }
+    return false;
+}
+
 DEV float3 node_lo(const DevEdgeNode &n) { return f3(n.lo[0], n.lo[1], n.lo[2]); }
 DEV float3 node_hi(const DevEdgeNode &n) { return f3(n.hi[0], n.hi[1], n.hi[2]); }
 DEV_NOINLINE float bsdf_bound(const DevEdgeNode &node, const BoundCtx &c, float *fast_m = nullptr) {
@@ -355,6 +412,12 @@ DEV_NOINLINE float bsdf_bound(const DevEdgeNode &node, const BoundCtx &c, float 
 DEV float3 sphere_center(float3 lo, float3 hi) {
     return f3((lo.x + hi.x) / 2.f, (lo.y + hi.y) / 2.f, (lo.z + hi.z) / 2.f);
 }
+DEV_NOINLINE bool cone_reaches_exact(float vt, float c, float a) {
+    float va = dr_atanf(vt);
+    float ang = dr_acosf(c);
+    float range = a + va;
+    return ang - range <= float(3.14159265358979323846 / 2.f) && ang + range >= float(3.14159265358979323846 / 2.f);
+}
 DEV bool cone_reaches_silhouette(float3 cs, float r, float3 axis, float a, float sa, float ca, float3 p) {
     float3 d = cs - p;
     float l = length(d);
@@ -373,10 +436,7 @@ DEV bool cone_reaches_silhouette(float3 cs, float r, float3 axis, float a, float
             if (ac > sin_r + margin) return false;
         }
     }
-    float va = dr_atanf(vt);
-    float ang = dr_acosf(c);
-    float range = a + va;
-    return ang - range <= float(3.14159265358979323846 / 2.f) && ang + range >= float(3.14159265358979323846 / 2.f);
+    return cone_reaches_exact(vt, c, a);
 }
 DEV_NOINLINE bool contains_silhouette(const DevEdgeNode &node, float3 p) {
     const float3 hi = node_hi(node), cs = sphere_center(node_lo(node), hi);
