@@ -29,7 +29,7 @@
 // taking runs of 2, 4 or 8 samples (7.1 ms with 8: neighbouring samples no
 // longer share their nodes' cache lines across the warp), 6 and 7 blocks per SM.
 #define DR_CONNECT_STACK 20  // deeper entries (up to DR_WIDE_STACK) go to local memory
-__global__ void __launch_bounds__(128, DR_CONNECT_BLOCKS) k_edge_connect(DevScene s, BackwardWorkspace ws) {
+__global__ void __launch_bounds__(128, DR_CONNECT_BLOCKS) k_edge_connect(const __grid_constant__ DevScene s, BackwardWorkspace ws) {
     __shared__ int stack[DR_CONNECT_STACK][128];
     int deep[DR_WIDE_STACK - DR_CONNECT_STACK];
     const long long n = (long long)min(ws.counters->survivors, (unsigned long long)ws.cap_items);

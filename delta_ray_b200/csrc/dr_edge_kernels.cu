@@ -103,7 +103,7 @@ __device__ __forceinline__ void add_visits(unsigned long long *counter, int visi
 }
 
 template <bool PROP>
-__global__ void __launch_bounds__(128, 6) k_edge_traverse(DevScene s, uint64_t seed, BackwardWorkspace ws) {
+__global__ void __launch_bounds__(128, 6) k_edge_traverse(const __grid_constant__ DevScene s, uint64_t seed, BackwardWorkspace ws) {
     const long long m = strided_points(ws);
     long long stride = (long long)gridDim.x * blockDim.x;
     ItemWriter out(ws);
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(128, 6) k_edge_traverse(DevScene s, uint64_t s
 #define DR_TASK_CUT 8
 #define DR_TASK_BUF 8
 template <bool PROP>
-__global__ void __launch_bounds__(128, 4) k_edge_expand(DevScene s, uint64_t seed, BackwardWorkspace ws) {
+__global__ void __launch_bounds__(128, 4) k_edge_expand(const __grid_constant__ DevScene s, uint64_t seed, BackwardWorkspace ws) {
     const long long m = strided_points(ws);
     long long stride = (long long)gridDim.x * blockDim.x;
     ItemWriter out(ws);
@@ -203,7 +203,7 @@ __device__ __forceinline__ long long next_task(unsigned long long *counter) {
 // `hand_q` (*hand_n) for the next round, so that no lane walks a long subtree
 // alone at the end of the launch.  The last round hands nothing on.
 template <bool PROP, bool HAND>
-__global__ void __launch_bounds__(128, DR_TASKS_BLOCKS) k_edge_tasks(DevScene s, uint64_t seed, BackwardWorkspace ws,
+__global__ void __launch_bounds__(128, DR_TASKS_BLOCKS) k_edge_tasks(const __grid_constant__ DevScene s, uint64_t seed, BackwardWorkspace ws,
                                                                    const EdgeTask *in, const unsigned long long *in_n,
                                                                    EdgeTask *hand_q, unsigned long long *hand_n) {
     const long long n = (long long)min(*in_n, (unsigned long long)ws.cap_tasks);
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(128, DR_TASKS_BLOCKS) k_edge_tasks(DevScene s,
 // draw picks (traverse_edges: edge_tree.cpp:685-725), that tree's probability
 // and whether its root splits the all walk.
 template <bool PROP>
-__global__ void __launch_bounds__(128, 8) k_walk_ctx(DevScene s, uint64_t seed, BackwardWorkspace ws) {
+__global__ void __launch_bounds__(128, 8) k_walk_ctx(const __grid_constant__ DevScene s, uint64_t seed, BackwardWorkspace ws) {
     const long long m = strided_points(ws);
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < m; k += stride) {
@@ -370,7 +370,7 @@ __device__ __forceinline__ void finish_item(const DevScene &s, const BackwardWor
 #include "dr_edge_connect.cuh"
 
 template <bool DIRECT>
-__global__ void __launch_bounds__(128, 4) k_edge_pairs(DevScene s, BackwardWorkspace ws) {
+__global__ void __launch_bounds__(128, 4) k_edge_pairs(const __grid_constant__ DevScene s, BackwardWorkspace ws) {
     const long long n = (long long)min(ws.counters->cands, (unsigned long long)ws.cap_items);
     while (true) {
         const long long j = next_task(&ws.counters->pair_next);
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(128, 4) k_edge_pairs(DevScene s, BackwardWorks
 // one slot (hits[slot].x = slot), which k_edge_shade reads as it does the
 // records of the ray stage.
 template <bool EXT, bool DIRECT>
-__global__ void __launch_bounds__(128, 8) k_edge_line_rays(DevScene s, uint64_t seed, BackwardWorkspace ws) {
+__global__ void __launch_bounds__(128, 8) k_edge_line_rays(const __grid_constant__ DevScene s, uint64_t seed, BackwardWorkspace ws) {
     long long n = (long long)min(ws.counters->items, (unsigned long long)ws.cap_items);
     long long stride = (long long)gridDim.x * blockDim.x;
     // warp-uniform loop: the append is warp-aggregated
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(128, 8) k_edge_line_rays(DevScene s, uint64_t 
 // multi-bounce shading) in a kernel of its own, [2 h] and [2 h + 1] of
 // ws.side_rad; k_edge_shade then runs without the path-tracing code, whose
 // size made the fused kernel wait on instruction fetches.
-__global__ void __launch_bounds__(128, DR_RADIANCE_BLOCKS) k_edge_radiance(DevScene s, int B, uint64_t seed,
+__global__ void __launch_bounds__(128, DR_RADIANCE_BLOCKS) k_edge_radiance(const __grid_constant__ DevScene s, int B, uint64_t seed,
                                                                     BackwardWorkspace ws) {
     long long n = (long long)min(ws.counters->cands, (unsigned long long)ws.cap_items);
     for (long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x; h < n; h += (long long)gridDim.x * blockDim.x) {
@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(128, DR_RADIANCE_BLOCKS) k_edge_radiance(DevSc
 
 // PRE: the sides' radiance comes from k_edge_radiance.
 template <bool EXT, bool GI, bool PRE>
-__global__ void __launch_bounds__(128, 4) k_edge_shade(DevScene s, int W, int H, int spp, int B, uint64_t seed,
+__global__ void __launch_bounds__(128, 4) k_edge_shade(const __grid_constant__ DevScene s, int W, int H, int spp, int B, uint64_t seed,
                                                     int dp_mode, float *grad, BackwardWorkspace ws, GradCacheCfg cfg) {
     extern __shared__ float sm[];
     BlockGrad bg = block_grad_begin(sm, grad, cfg);
@@ -504,13 +504,13 @@ __global__ void __launch_bounds__(128, 4) k_edge_shade(DevScene s, int W, int H,
 // code of a forward path), k_primary_grad redraws the sample and turns the
 // color difference into the scene and camera gradients.
 template <int BMAX>
-__global__ void __launch_bounds__(128, 6) k_primary_shade(DevScene s, int B, uint64_t seed, long long i0, long long n,
+__global__ void __launch_bounds__(128, 6) k_primary_shade(const __grid_constant__ DevScene s, int B, uint64_t seed, long long i0, long long n,
                                                        float4 *out) {
     for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
         out[k] = primary_shade_item<BMAX>(s, i0 + k, B, seed);
 }
 
-__global__ void __launch_bounds__(128, 8) k_primary_grad(DevScene s, int W, int H, int spp, uint64_t seed,
+__global__ void __launch_bounds__(128, 8) k_primary_grad(const __grid_constant__ DevScene s, int W, int H, int spp, uint64_t seed,
                                                       const float *d_image, long long i0, long long n,
                                                       const float4 *in, float *grad, GradCacheCfg cfg) {
     extern __shared__ float sm[];
@@ -532,7 +532,7 @@ cudaError_t dr_launch_accumulate_count(unsigned long long *dst, const unsigned l
     return cudaGetLastError();
 }
 
-__global__ void k_edge_records(DevScene s, const DevEdge *edges, int n, EdgeRec *out) {
+__global__ void k_edge_records(const __grid_constant__ DevScene s, const DevEdge *edges, int n, EdgeRec *out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = edge_record(s, edges[i]);
 }
@@ -727,7 +727,7 @@ cudaError_t dr_launch_primary_edges(const DevScene &s, int W, int H, int spp, in
 
 // The learned proposal's inputs of each shading point: position normalised to
 // the scene bounds, shading normal, roughness, incoming direction.
-__global__ void k_proposal_features(DevScene s, BackwardWorkspace ws, long long n, float3 c, float3 ih,
+__global__ void k_proposal_features(const __grid_constant__ DevScene s, BackwardWorkspace ws, long long n, float3 c, float3 ih,
                                     __nv_bfloat16 *x, __nv_bfloat16 *xt) {
     long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;

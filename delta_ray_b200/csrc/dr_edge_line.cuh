@@ -11,7 +11,7 @@
 // lobe mixture weight): 6-8 the other lobe's transform and its pick
 // probability.
 template <bool MIS>
-__global__ void __launch_bounds__(128, 8) k_line_ctx(DevScene s, uint64_t seed, BackwardWorkspace ws) {
+__global__ void __launch_bounds__(128, 8) k_line_ctx(const __grid_constant__ DevScene s, uint64_t seed, BackwardWorkspace ws) {
     const long long n = min(min((long long)ws.counters->points, ws.cap_points), ws.pt_end);
     for (long long p = ws.pt_begin + (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
          p += (long long)gridDim.x * blockDim.x) {
@@ -71,7 +71,7 @@ enum { kItem, kU, kVoX, kVoY, kVoZ, kWtX, kWtY, kWtZ, kD, kIl0, kNorm, kL0, kL1 
 // items), 5.5 -> 2.6 at 160x120; with the lobe mixture weight on a 64x64-vertex
 // heightfield (15.5 M items) 5.4 -> 2.6.  21 of 32 lanes active.
 template <bool MIS>
-__global__ void __launch_bounds__(128, DR_LINE_BLOCKS) k_edge_line(DevScene s, BackwardWorkspace ws) {
+__global__ void __launch_bounds__(128, DR_LINE_BLOCKS) k_edge_line(const __grid_constant__ DevScene s, BackwardWorkspace ws) {
     __shared__ LineTile block_tile[4];
     LineTile &t = block_tile[threadIdx.x >> 5];
     const unsigned full = 0xffffffffu;
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(128, DR_LINE_BLOCKS) k_edge_line(DevScene s, B
 // holds none): one lane per item, the setup per edge.  EXT:
 // DR_FLAG_EDGE_LOBE_MIS or proposal training in use.
 template <bool EXT>
-__global__ void __launch_bounds__(128, 4) k_edge_line_point(DevScene s, uint64_t seed, BackwardWorkspace ws) {
+__global__ void __launch_bounds__(128, 4) k_edge_line_point(const __grid_constant__ DevScene s, uint64_t seed, BackwardWorkspace ws) {
     const long long n = (long long)min(ws.counters->items, (unsigned long long)ws.cap_items);
     const long long stride = (long long)gridDim.x * blockDim.x;
     // warp-uniform loop: the survivor append is warp-aggregated

@@ -149,7 +149,7 @@ template <bool PROP> struct WalkWarp {
 // warps spread it; the last round (out == null) walks to the end.
 
 template <bool PROP>
-__global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(DevScene s, BackwardWorkspace ws, int round,
+__global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_constant__ DevScene s, BackwardWorkspace ws, int round,
                                                                  const WalkPacket *in, WalkPacket *out) {
     __shared__ WalkWarp<PROP> block_sh[4];
     WalkWarp<PROP> &sh = block_sh[threadIdx.x >> 5];

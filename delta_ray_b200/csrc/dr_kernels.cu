@@ -176,7 +176,7 @@ cudaError_t dr_widen_lbvh(const float4 *nodes, int n, float4 *wide, cudaStream_t
     return cudaGetLastError();
 }
 
-__global__ void k_trace_rays(DevScene s, const float *rays, long long n, int *tri, float *t) {
+__global__ void k_trace_rays(const __grid_constant__ DevScene s, const float *rays, long long n, int *tri, float *t) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float *r = rays + 6 * i;
@@ -208,7 +208,7 @@ cudaError_t dr_launch_trace(const DevScene &s, const float *rays, long long n, i
 // Forward render: one pixel sample per (pixel, lane) and a segmented warp
 // reduction over the 2^lanes_log2 lanes of a pixel.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256, 4) k_render_forward(DevScene s, int W, int H, int spp, int B, uint64_t seed,
+__global__ void __launch_bounds__(256, 4) k_render_forward(const __grid_constant__ DevScene s, int W, int H, int spp, int B, uint64_t seed,
                                                         int lanes_log2, float *img) {
     long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int G = 1 << lanes_log2;

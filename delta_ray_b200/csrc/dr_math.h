@@ -32,8 +32,10 @@
 
 #if defined(__CUDACC__)
 #define DRM_FN __host__ __device__ __forceinline__
+#define DRM_OUT static __host__ __device__ __noinline__
 #else
 #define DRM_FN inline
+#define DRM_OUT inline
 #endif
 
 namespace drm {
@@ -420,9 +422,9 @@ DRM_FN float dr_acosf(float x) {
     if (x == -1.f) return drm::kPiHf;
     return drm::fmul(2.f, drm::atanf_pos(drm::froot(drm::fdiv(drm::fsub(1.f, x), drm::fadd(1.f, x)))));
 }
-DRM_FN float dr_expf(float x) { return (float)drm::exp_d((double)x); }
-DRM_FN float dr_logf(float x) { return (float)drm::log_d((double)x); }
-DRM_FN float dr_powf(float x, float y) { return (float)drm::pow_d((double)x, (double)y); }
+DRM_OUT float dr_expf(float x) { return (float)drm::exp_d((double)x); }
+DRM_OUT float dr_logf(float x) { return (float)drm::log_d((double)x); }
+DRM_OUT float dr_powf(float x, float y) { return (float)drm::pow_d((double)x, (double)y); }
 
 // Dispatch by function number (0 sin, 1 cos, 2 atan, 3 atan2(x, y), 4 acos,
 // 5 exp, 6 log, 7 pow(x, y)): the check hooks of the library and of the host
