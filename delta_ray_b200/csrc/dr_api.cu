@@ -95,7 +95,35 @@ struct EdgeStats {
     DevBuf dev;                               // the reduction's output
 };
 
+// Streams beside a call's own on which the front stages of a batch of views
+// run at once, forked from the call's stream and joined to it by events.
+struct SideStreams {
+    static constexpr int kMax = 8;
+    int n = 0;
+    cudaStream_t s[kMax];
+    cudaEvent_t done[kMax], fork = nullptr;
+    void need(int want) {
+        want = std::min(want, kMax);
+        if (!fork) check_cuda(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "cudaEventCreate");
+        while (n < want) {
+            check_cuda(cudaStreamCreateWithFlags(&s[n], cudaStreamNonBlocking), "cudaStreamCreate");
+            cudaError_t e = cudaEventCreateWithFlags(&done[n], cudaEventDisableTiming);
+            if (e != cudaSuccess) cudaStreamDestroy(s[n]);
+            check_cuda(e, "cudaEventCreate");
+            n++;
+        }
+    }
+    ~SideStreams() {
+        for (int i = 0; i < n; i++) {
+            cudaEventDestroy(done[i]);
+            cudaStreamDestroy(s[i]);
+        }
+        if (fork) cudaEventDestroy(fork);
+    }
+};
+
 struct BackwardQueues {
+    SideStreams side;
     DevBuf pt, items, item_w, item_dp, pt_last, pt_items, counts, survivors, hits, side_rad, tasks, tasks2;
     DevBuf walk_ctx, packets;  // the warp walk: the points' contexts, its rounds' packets
     DevBuf line_ctx;         // the points' line-sample setups
@@ -657,7 +685,7 @@ std::pair<long long, long long> run_backward(dr_scene *scene, const dr_render_de
                                              cudaStream_t st, StageTimer *timer, Grow grow, GrowPoints grow_points,
                                              ProposalState *prop = nullptr, const DevScene *view = nullptr,
                                              EdgeStats *stats = nullptr, const std::vector<FrontCall> *fronts = nullptr,
-                                             long long grad_len = 0) {
+                                             long long grad_len = 0, SideStreams *side = nullptr) {
     const DevScene ds = fronts ? (*fronts)[0].ds : view ? *view : call_scene(scene, rd);
     const GradCacheCfg cfg = grad_cache_cfg(scene->h);
     BackwardCounters c;
@@ -745,14 +773,45 @@ std::pair<long long, long long> run_backward(dr_scene *scene, const dr_render_de
         ws.pt_begin = 0;
         ws.pt_end = ws.cap_points;
         if (fronts) {
+            // The views' front stages at once, on streams of their own: one
+            // view's launch is often too small to fill the GPU, and takes as
+            // long as its slowest warp (six views of 25,000 samples of a room
+            // 12.8 ms in turn).  Each view's primary edges get a part of the
+            // item queue for their color differences; in turn where it has no
+            // room for all, and under the stage timer, which times a stream.
+            std::vector<long long> part(fronts->size() + 1, 0);
             for (size_t k = 0; k < fronts->size(); k++) {
-                const FrontCall &f = (*fronts)[k];
-                check_launch(dr_launch_backward_front(f.ds, f.rd.width, f.rd.height, f.rd.spp, f.rd.max_bounces,
-                                                      f.rd.seed, f.d_image, grad_dev, f.image,
-                                                      f.rd.primary_edge_samples, f.rd.dp_mode, ws, cfg,
-                                                      scene->num_sms, st, &scene->last_launches, timer, false, k == 0),
-                             "backward launch");
+                const dr_render_desc &r = (*fronts)[k].rd;
+                part[k + 1] = part[k] + (r.primary_edge_samples > 0 ? (long long)r.primary_edge_samples
+                                                                    : (long long)r.spp * r.width * r.height);
             }
+            const bool at_once = side && !timer->on && !timer->sync && part.back() <= ws.cap_items;
+            if (at_once) {
+                side->need((int)fronts->size());
+                check_cuda(cudaEventRecord(side->fork, st), "fork");
+                for (int i = 0; i < side->n; i++) check_cuda(cudaStreamWaitEvent(side->s[i], side->fork, 0), "fork");
+            }
+            cudaError_t launched = cudaSuccess;
+            for (size_t k = 0; k < fronts->size() && launched == cudaSuccess; k++) {
+                const FrontCall &f = (*fronts)[k];
+                BackwardWorkspace wv = ws;
+                if (at_once) {
+                    wv.items += part[k];
+                    wv.cap_items = part[k + 1] - part[k];
+                }
+                launched = dr_launch_backward_front(f.ds, f.rd.width, f.rd.height, f.rd.spp, f.rd.max_bounces, f.rd.seed,
+                                                    f.d_image, grad_dev, f.image, f.rd.primary_edge_samples,
+                                                    f.rd.dp_mode, wv, cfg, scene->num_sms,
+                                                    at_once ? side->s[k % side->n] : st, &scene->last_launches, timer,
+                                                    false, k == 0);
+            }
+            if (at_once) {  // joined on every way out, so that the queues are idle when st is
+                for (int i = 0; i < side->n; i++) {
+                    check_cuda(cudaEventRecord(side->done[i], side->s[i]), "join");
+                    check_cuda(cudaStreamWaitEvent(st, side->done[i], 0), "join");
+                }
+            }
+            check_launch(launched, "backward launch");
         } else {
             check_launch(dr_launch_backward_front(ds, rd->width, rd->height, rd->spp, rd->max_bounces, rd->seed,
                                                   d_image_dev, grad_dev, image_dev, rd->primary_edge_samples,
@@ -1195,7 +1254,7 @@ void backward_on_queues(dr_scene *scene, const dr_render_desc *rd, const DevScen
     }
     ws.views = views_dev;
     auto counts = run_backward(scene, rd, d_image_dev, grad_dev, image_dev, ws, st, &scene->timer, grow, grow_points,
-                               prop, view, &q.stats, fronts, grad_len);
+                               prop, view, &q.stats, fronts, grad_len, &q.side);
     scene->last_points = counts.first;
     scene->last_items = counts.second;
 }

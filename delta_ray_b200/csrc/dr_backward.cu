@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(128, 8) k_backward_paths(const __grid_constant
                                                         int lanes_log2, const float *d_image, float *grad, float *img,
                                                         BackwardWorkspace ws, GradCacheCfg cfg) {
     extern __shared__ float sm[];
-    BlockGradWarp bg;
+    PathGrad<kChains> bg;
     static_cast<BlockGrad &>(bg) = block_grad_begin(sm, grad, cfg);
     long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int G = 1 << lanes_log2;
@@ -94,7 +94,7 @@ template <bool kChains>
 __global__ void __launch_bounds__(128, 6) k_dp_propagate(const __grid_constant__ DevScene s, int W, int H, int spp, uint64_t seed, int dp_mode,
                                                       float *grad, BackwardWorkspace ws, GradCacheCfg cfg) {
     extern __shared__ float sm[];
-    BlockGradWarp bg;
+    PathGrad<kChains> bg;
     static_cast<BlockGrad &>(bg) = block_grad_begin(sm, grad, cfg);
     long long n = min(min((long long)ws.counters->points, ws.cap_points), ws.pt_end);
     for (long long p = ws.pt_begin + (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
@@ -135,7 +135,7 @@ cudaError_t dr_launch_backward_front(const DevScene &s, int W, int H, int spp, i
     int lanes_log2 = path_lanes_log2(spp);
     long long threads = ((long long)W * H) << lanes_log2;
     if (first) timer->begin(st);  // a later view's front stage of a batched call continues the timing
-    if (dp_mode != DR_DP_SUM || s.specular_chains) {
+    if (first && (dp_mode != DR_DP_SUM || s.specular_chains)) {
         // LAST: one key per point; SUM with chains: a float4 dp sum per point
         size_t per = dp_mode == DR_DP_SUM ? DR_PT_LAST_BYTES : sizeof(unsigned long long);
         cudaError_t e = cudaMemsetAsync(ws.pt_last, 0, per * (size_t)ws.cap_points, st);

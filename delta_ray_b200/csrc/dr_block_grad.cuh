@@ -37,6 +37,36 @@ struct BlockGradWarp : BlockGrad {
     }
 };
 
+// The same for kernels whose warps run in parts (paths through specular chains:
+// 13 of 32 lanes active): the active lanes that add to one entry sum with
+// shuffles, as many rounds as the largest group has lanes, and add once.  Lanes
+// adding to one shared entry one after another made a launch of 25,000 samples
+// in a room of 12 spheres take 3.2 ms, 2.1 with this; where most adds are a
+// full warp's to one entry the plain form is the faster one (k_primary_grad on
+// the soft shadow 1.37 against 1.76 ms).
+struct BlockGradGroups : BlockGrad {
+    __device__ __forceinline__ void add(int i, float v) {
+        const unsigned mask = __activemask();
+        const unsigned peers = __match_any_sync(mask, i);
+        if (peers == 0xffffffffu) {
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        } else {
+            float sum = 0.f;
+            unsigned m = peers;
+            do {
+                const float t = __shfl_sync(mask, v, m ? __ffs(m) - 1 : (int)(threadIdx.x & 31));
+                if (m) sum += t;
+                m &= m - 1;
+            } while (__any_sync(mask, m != 0));
+            v = sum;
+        }
+        if ((int)(threadIdx.x & 31) != __ffs(peers) - 1) return;
+        BlockGrad::add(i, v);
+    }
+};
+template <bool kChains> struct PathGrad : BlockGradWarp {};
+template <> struct PathGrad<true> : BlockGradGroups {};
+
 __device__ __forceinline__ BlockGrad block_grad_begin(float *sm, float *g, const GradCacheCfg &c) {
     BlockGrad b;
     b.sm = sm;
