@@ -654,16 +654,15 @@ DEV bool item_line(const DevScene &s, const PointRecord &pt, int tree, int ei, u
 
 // The item's shading from its line sample; as eval_item.  `hits` (may be
 // null): the closest hits of the sample's two rays, which edge_rays kept.
-// The two sides' radiance of a kept edge sample (edge_side_radiance), with
+// The radiance of one side of a kept edge sample (edge_side_radiance), with
 // the item's own light sample and random stream as item_shade draws them.
-DEV bool item_side_radiance(const DevScene &s, const PointRecord &pt, int tree, int ei, int j, int B,
-                            uint64_t seed, const EdgeLine &el, const EdgeHits &hits, float3 &shr, float3 &shl) {
+DEV float3 item_side_radiance(const DevScene &s, const PointRecord &pt, int tree, int ei, int j, int B,
+                              uint64_t seed, const EdgeLine &el, int tri, int k) {
     Rng irng;
     irng.init(seed, kStreamEdgeItem, pt.sid, ((uint32_t)pt.bounce << 28) | (uint32_t)j);
     LightSample els = draw_light(irng);
-    const DevEdge &edge = tree ? s.nrm_edges[ei] : s.sil_edges[ei];
-    return edge_side_radiance(s, el, edge, els, irng, B - pt.bounce - 1, pt.wi, pt.tri, pt.surface(), hits, shr,
-                              shl);
+    return edge_side_radiance(s, el, (tree ? s.nrm_rec : s.sil_rec) + ei, els, irng, B - pt.bounce - 1, pt.wi, pt.tri,
+                              pt.surface(), tri, k);
 }
 
 // PRE: the sides' radiance `rad` comes from item_side_radiance (see

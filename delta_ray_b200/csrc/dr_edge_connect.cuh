@@ -19,13 +19,13 @@
 // way: samples follow each other by edge, and at the 130,054-triangle
 // heightfield a blocker of the sample before blocks about half of the occluded
 // right rays, the right ray's four in five of the left rays beside it, and a
-// walk saved is about 45 nodes.  Any blocking triangle gives the walk's answer,
-// as long as it lies clearly ahead of the face (by 1e-3 of the distance):
-// nearer, the walk's box tests and the triangle test may round to different
-// sides, and only the walk decides.  The walk's stack lies in shared memory, a
+// walk saved is about 45 nodes.  Any triangle that the walk would test and
+// that blocks gives its answer (leaf_entered).  The boxes are tested with fused
+// multiply-adds, which enter a few more than the walk's own test would.  The
+// walk's stack lies in shared memory, a
 // column per lane (in local memory it took as much of the L1's throughput as
-// the nodes).  Measured there: 99 -> 75 ms at 640x480, 1 spp (120 M samples),
-// 6.3 -> 4.8 at 160x120, 18 of 32 lanes active (14.7 before).  Dropped: lanes
+// the nodes).  Measured there: 99 -> 69.5 ms at 640x480, 1 spp (120 M samples),
+// 6.3 -> 4.5 at 160x120, 19 of 32 lanes active (14.7 before).  Dropped: lanes
 // taking runs of 2, 4 or 8 samples (7.1 ms with 8: neighbouring samples no
 // longer share their nodes' cache lines across the warp), 6 and 7 blocks per SM.
 #define DR_CONNECT_STACK 20  // deeper entries (up to DR_WIDE_STACK) go to local memory
@@ -33,11 +33,12 @@ __global__ void __launch_bounds__(128, DR_CONNECT_BLOCKS) k_edge_connect(const _
     __shared__ int stack[DR_CONNECT_STACK][128];
     int deep[DR_WIDE_STACK - DR_CONNECT_STACK];
     const long long n = (long long)min(ws.counters->survivors, (unsigned long long)ws.cap_items);
-    const float tnear = 1e-3f, kAhead = 1.f - 1e-3f;
+    const float tnear = 1e-3f;
     long long k = 0;  // the lane's sample
     int phase = 0;  // 0 no walk, 1 walking the right ray, 2 walking the left ray
     bool more = true, cr = false;
-    float3 p = f3(0.f), d = f3(0.f), inv = f3(0.f), ldir = f3(0.f);
+    float3 p = f3(0.f), d = f3(0.f), ldir = f3(0.f);
+    FastRay ray = fast_ray(f3(0.f), f3(1.f));
     int r_tri = -1, l_tri = -1, node = 0, sp = 0, leaf = -1, blocker = -1;
     float l_t = 0.f, ta = 0.f;
     int ida = -1;
@@ -55,11 +56,13 @@ __global__ void __launch_bounds__(128, DR_CONNECT_BLOCKS) k_edge_connect(const _
         const float4 a = __ldg(s.bvh_tris + 3 * leaf), b = __ldg(s.bvh_tris + 3 * leaf + 1),
                      c = __ldg(s.bvh_tris + 3 * leaf + 2);
         float t;
-        return hit_triangle(a, b, c, p, dir, t) && t > tnear && (t < t_face || (t == t_face && __float_as_int(a.w) < face));
+        return hit_triangle(a, b, c, p, dir, t) && t > tnear &&
+               (t < t_face || (t == t_face && __float_as_int(a.w) < face)) &&
+               leaf_entered(a, b, c, p, f3(safe_inv(dir.x), safe_inv(dir.y), safe_inv(dir.z)), t_face);
     };
     const auto begin = [&](int ph, float3 dir, float t_face, int face) {
         d = dir;
-        inv = f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+        ray = fast_ray(p, f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z)));
         ta = t_face;
         ida = face;
         sp = 0;
@@ -77,7 +80,7 @@ __global__ void __launch_bounds__(128, DR_CONNECT_BLOCKS) k_edge_connect(const _
         phase = 0;
         if (l_tri < 0) {
             if (cr) candidate(0, r_tri);
-        } else if (blocker >= 0 && blocks(blocker, ldir, l_t * kAhead, l_tri)) {
+        } else if (blocker >= 0 && blocks(blocker, ldir, l_t, l_tri)) {
             if (cr) candidate(0, r_tri);
         } else {
             begin(2, ldir, l_t, l_tri);
@@ -109,7 +112,7 @@ __global__ void __launch_bounds__(128, DR_CONNECT_BLOCKS) k_edge_connect(const _
             l_tri = fl.tri;
             l_t = fl.t;
             cr = false;
-            if (r_tri >= 0 && !(blocker >= 0 && blocks(blocker, rdir, fr.t * kAhead, fr.tri))) begin(1, rdir, fr.t, fr.tri);
+            if (r_tri >= 0 && !(blocker >= 0 && blocks(blocker, rdir, fr.t, fr.tri))) begin(1, rdir, fr.t, fr.tri);
             else after_right();
         }
         if (fetch) continue;
@@ -123,13 +126,17 @@ __global__ void __launch_bounds__(128, DR_CONNECT_BLOCKS) k_edge_connect(const _
         int res = 0;  // 1 a triangle ahead, 2 none, 0 not known yet
         if (2 * __popc(inner) >= __popc(walking)) {
             if (phase != 0 && node >= 0 && node != DR_WIDE_EMPTY) {
-                const WideKids kids = wide_kids(s.bvh_wide + (size_t)DR_WIDE_F4 * node, p, inv, ta);
-                if (kids.n == 0) {
+                const FastKids kids = fast_kids(s.bvh_wide + (size_t)DR_WIDE_F4 * node, ray, ta);
+                if (!kids.any) {
                     node = sp > 0 ? pop() : DR_WIDE_EMPTY;
                 } else {
-                    if (kids.n > 3) push(kids.c[3]);
-                    if (kids.n > 2) push(kids.c[2]);
-                    if (kids.n > 1) push(kids.c[1]);
+                    if (sp <= DR_CONNECT_STACK - 3) {
+                        for (int i = 3; i > 0; i--)
+                            if (kids.hit[i]) stack[sp++][threadIdx.x] = kids.c[i];
+                    } else {
+                        for (int i = 3; i > 0; i--)
+                            if (kids.hit[i]) push(kids.c[i]);
+                    }
                     node = kids.c[0];
                 }
                 if (node < 0 && leaf < 0) {

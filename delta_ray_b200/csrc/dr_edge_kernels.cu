@@ -433,29 +433,25 @@ __global__ void __launch_bounds__(128, 8) k_edge_line_rays(const __grid_constant
 
 // More than one bounce: the two sides' radiance of every kept sample (the
 // multi-bounce shading) in a kernel of its own, [2 h] and [2 h + 1] of
-// ws.side_rad; k_edge_shade then runs without the path-tracing code, whose
-// size made the fused kernel wait on instruction fetches.
-__global__ void __launch_bounds__(128, DR_RADIANCE_BLOCKS) k_edge_radiance(const __grid_constant__ DevScene s, int B, uint64_t seed,
-                                                                    BackwardWorkspace ws) {
-    long long n = (long long)min(ws.counters->cands, (unsigned long long)ws.cap_items);
-    for (long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x; h < n; h += (long long)gridDim.x * blockDim.x) {
-        int4 hr = ws.hits[h];
+// ws.side_rad, one lane per side; k_edge_shade then runs without the
+// path-tracing code, whose size made the fused kernel wait on instruction
+// fetches.
+__global__ void __launch_bounds__(128, DR_RADIANCE_BLOCKS) k_edge_radiance(const __grid_constant__ DevScene s, int B,
+                                                                         uint64_t seed, BackwardWorkspace ws) {
+    const long long n = 2 * (long long)min(ws.counters->cands, (unsigned long long)ws.cap_items);
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const int k = (int)(q & 1);
+        const int4 hr = ws.hits[q >> 1];
         if (hr.w == 0) continue;
-        EdgeHits eh;
-        eh.r = hr.y;
-        eh.l = hr.z;
-        float4 a = ws.survivors[2 * (long long)hr.x];
-        long long i = __float_as_int(a.x);
+        const float4 a = ws.survivors[2 * (long long)hr.x];
         EdgeLine el;
         el.sample_p = f3(a.y, a.z, a.w);
-        int4 it = ws.items[i];
+        const int4 it = ws.items[__float_as_int(a.x)];
         PointRecord pt;
         pt.load(ws.pt + (size_t)it.x * DR_PT_WORDS);
-        float3 shr, shl;
-        item_side_radiance(s, pt, it.y >> 30, it.y & ((1 << 30) - 1), it.z, B, point_seed(ws, pt.view, seed), el, eh,
-                           shr, shl);
-        ws.side_rad[2 * h] = make_float4(shr.x, shr.y, shr.z, shl.x);
-        ws.side_rad[2 * h + 1] = make_float4(shl.y, shl.z, 0.f, 0.f);
+        const float3 r = item_side_radiance(s, pt, it.y >> 30, it.y & ((1 << 30) - 1), it.z, B,
+                                            point_seed(ws, pt.view, seed), el, k ? hr.z : hr.y, k);
+        ws.side_rad[q] = make_float4(r.x, r.y, r.z, 0.f);
     }
 }
 
@@ -488,7 +484,7 @@ __global__ void __launch_bounds__(128, 4) k_edge_shade(const __grid_constant__ D
         float3 dp;
         if constexpr (PRE) {
             const float4 r0 = ws.side_rad[2 * h], r1 = ws.side_rad[2 * h + 1];
-            const float3 rad[2] = {f3(r0.x, r0.y, r0.z), f3(r0.w, r1.x, r1.y)};
+            const float3 rad[2] = {f3(r0.x, r0.y, r0.z), f3(r1.x, r1.y, r1.z)};
             dp = item_shade<EXT, GI, BlockGrad, true>(s, pt, tree, ei, it.z, ws.item_w[i], v.spp, B, v.seed, bg, &mag,
                                                      el, &eh, rad);
         } else {

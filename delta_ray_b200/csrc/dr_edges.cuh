@@ -1333,34 +1333,22 @@ DEV bool edge_rays(const DevScene &s, const EdgeLine &el, const DevEdge &edge, c
 // (with more bounces) the radiance seen on each side, the BSDF toward the
 // edge, and the Jacobians of the sample w.r.t. the shading point and the
 // edge's end points.
-// The radiance each side of an edge sample receives beyond its closest hit
-// (more bounces than one), divided by the squared distance and times the
-// cosine at the hit, as edge_shade_hits uses it; false (and zeros) when the
-// BSDF toward the edge is negligible, where edge_shade_hits ends the sample.
-DEV bool edge_side_radiance(const DevScene &s, const EdgeLine &el_, const DevEdge &edge, const LightSample &ls,
-                            const Rng &rng, int nbounces, float3 wi, int stri, const SurfacePoint &sp,
-                            const EdgeHits &hits, float3 &shr, float3 &shl) {
-    shr = shl = f3(0.f);
-    float3 v0 = edge_v0(s, edge), v1 = edge_v1(s, edge);
+// The radiance side k (0 right, 1 left) of an edge sample receives beyond its
+// closest hit (more bounces than one), divided by the squared distance and
+// times the cosine at the hit, as edge_shade_hits uses it; zero where the BSDF
+// toward the edge is negligible, where edge_shade_hits ends the sample.
+DEV float3 edge_side_radiance(const DevScene &s, const EdgeLine &el_, const EdgeRec *rec, const LightSample &ls,
+                              const Rng &rng, int nbounces, float3 wi, int stri, const SurfacePoint &sp, int tri,
+                              int k) {
+    if (tri < 0) return f3(0.f);
     float3 sdir, rdir, ldir;
-    edge_side_dirs(el_, v0, v1, sp.p, sdir, rdir, ldir);
-    if (sum(bsdf(s, material_of_tri(s, stri), sp, wi, sdir)) < 1e-6f) return false;
-#pragma unroll 1
-    for (int k = 0; k < 2; k++) {
-        int tri = k == 0 ? hits.r : hits.l;
-        SurfacePoint pp;
-        if (tri >= 0) pp = intersect_tri(load_tri(s, tri), sp.p, k == 0 ? rdir : ldir);
-        float3 sh = shade(s, -sdir, tri, pp, ls, rng, nbounces, false);
-        if (tri >= 0) {
-            float3 dir = pp.p - sp.p;
-            float d2 = length_sq(dir);
-            if (d2 > 0.f) sh = sh / fmaxf(d2, 1e-2f) * fabsf(dot(normalize(dir), pp.ng));
-            else sh = f3(0.f);
-        }
-        if (k == 0) shr = sh;
-        else shl = sh;
-    }
-    return true;
+    edge_side_dirs(el_, rec_v0(rec), rec_v1(rec), sp.p, sdir, rdir, ldir);
+    if (sum(bsdf(s, material_of_tri(s, stri), sp, wi, sdir)) < 1e-6f) return f3(0.f);
+    const SurfacePoint pp = intersect_tri(load_tri(s, tri), sp.p, k == 0 ? rdir : ldir);
+    const float3 sh = shade(s, -sdir, tri, pp, ls, rng, nbounces, false);
+    const float3 dir = pp.p - sp.p;
+    const float d2 = length_sq(dir);
+    return d2 > 0.f ? sh / fmaxf(d2, 1e-2f) * fabsf(dot(normalize(dir), pp.ng)) : f3(0.f);
 }
 
 // PRE: the two sides' radiance comes from edge_side_radiance, computed by an

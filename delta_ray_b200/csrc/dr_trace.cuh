@@ -439,6 +439,81 @@ DEV bool wide_next(const WideKids &k, int *stack, int &sp, int &node) {
     return true;
 }
 
+// A ray as the fast box tests take it: inv and -o inv, the latter below and
+// above its value by more than the tests' rounding.  A slab's distance is then
+// one fused multiply-add instead of a subtraction and a multiplication, and a
+// box that box_entry lets pass passes here too: the two distances differ by at
+// most 2^-22 |t| (allowed for where the bounds are compared) and 2^-23 |o inv|
+// (the offsets).  Which boxes a bounded walk enters decides nothing as long as
+// it enters those: the boxes of a leaf's ancestors contain its own, with the
+// same floats, and box_entry's rounded distances do not cross when a box
+// grows, so box_entry lets a leaf's ancestors pass whenever it lets its own box
+// pass (leaf_entered).  The walk over box_entry thus tests exactly the
+// triangles whose own boxes pass, in whatever order.
+struct FastRay {
+    float3 inv, near_off, far_off;
+};
+DEV FastRay fast_ray(float3 o, float3 inv) {
+    FastRay r;
+    r.inv = inv;
+    const float3 oi = f3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
+    const float3 pad = f3(fabsf(oi.x) * 4e-7f, fabsf(oi.y) * 4e-7f, fabsf(oi.z) * 4e-7f);
+    r.near_off = f3(-oi.x - pad.x, -oi.y - pad.y, -oi.z - pad.z);
+    r.far_off = f3(-oi.x + pad.x, -oi.y + pad.y, -oi.z + pad.z);
+    return r;
+}
+#ifdef DR_HOST_BUILD
+HD float fma_rn(float a, float b, float c) { return std::fma(a, b, c); }
+#else
+DEV float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+#endif
+// Entry distance (>= 0) of a child box of a wide node, from its near and far
+// planes; infinity on a miss.
+DEV float fast_entry(float nx, float ny, float nz, float fx, float fy, float fz, const FastRay &r, float tmax) {
+    const float tn = fmaxf(fmaxf(fma_rn(nx, r.inv.x, r.near_off.x), fma_rn(ny, r.inv.y, r.near_off.y)),
+                           fmaxf(fma_rn(nz, r.inv.z, r.near_off.z), 0.f));
+    const float tf = fminf(fminf(fma_rn(fx, r.inv.x, r.far_off.x), fma_rn(fy, r.inv.y, r.far_off.y)),
+                           fminf(fma_rn(fz, r.inv.z, r.far_off.z), tmax));
+    return tn <= tf * 1.000002f ? tn : DR_INF;
+}
+// The children of wide node w that the ray may enter before tmax: c[0] the
+// nearest (any says whether there is one) and c[i] where hit[i] is set.
+struct FastKids {
+    bool any, hit[4];
+    int c[4];
+};
+DEV FastKids fast_kids(const float4 *DR_RESTRICT w, const FastRay &r, float tmax) {
+    const int sx = r.inv.x < 0.f ? 3 : 0, sy = r.inv.y < 0.f ? 3 : 0, sz = r.inv.z < 0.f ? 3 : 0;
+    const float4 nx = dr_ldg(w + sx), ny = dr_ldg(w + 1 + sy), nz = dr_ldg(w + 2 + sz);
+    const float4 fx = dr_ldg(w + 3 - sx), fy = dr_ldg(w + 4 - sy), fz = dr_ldg(w + 5 - sz), rf = dr_ldg(w + 6);
+    int c0 = dr_f2i(rf.x), c1 = dr_f2i(rf.y), c2 = dr_f2i(rf.z), c3 = dr_f2i(rf.w);
+    float k0 = fast_entry(nx.x, ny.x, nz.x, fx.x, fy.x, fz.x, r, tmax);
+    float k1 = fast_entry(nx.y, ny.y, nz.y, fx.y, fy.y, fz.y, r, tmax);
+    float k2 = c2 != DR_WIDE_EMPTY ? fast_entry(nx.z, ny.z, nz.z, fx.z, fy.z, fz.z, r, tmax) : DR_INF;
+    float k3 = c3 != DR_WIDE_EMPTY ? fast_entry(nx.w, ny.w, nz.w, fx.w, fy.w, fz.w, r, tmax) : DR_INF;
+    wide_swap(k0, c0, k1, c1);
+    wide_swap(k2, c2, k3, c3);
+    wide_swap(k0, c0, k2, c2);
+    FastKids out;
+    out.any = k0 < DR_INF;
+    out.hit[0] = false;
+    out.hit[1] = k1 < DR_INF;
+    out.hit[2] = k2 < DR_INF;
+    out.hit[3] = k3 < DR_INF;
+    out.c[0] = c0;
+    out.c[1] = c1;
+    out.c[2] = c2;
+    out.c[3] = c3;
+    return out;
+}
+// Whether box_entry lets the triangle's own box pass before tmax (and so the
+// boxes around it, see FastRay).
+DEV bool leaf_entered(float4 a, float4 b, float4 c, float3 o, float3 inv, float tmax) {
+    return box_entry(fminf(fminf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y), fminf(fminf(a.z, b.z), c.z),
+                     fmaxf(fmaxf(a.x, b.x), c.x), fmaxf(fmaxf(a.y, b.y), c.y), fmaxf(fmaxf(a.z, b.z), c.z), o, inv,
+                     tmax) >= 0.f;
+}
+
 // The walk of trace_before_bvh as a resumable state: begin() sets it up,
 // step() takes one node (a box pair or a leaf) and returns 0 while the walk
 // goes on, 1 when a triangle hits ahead of (ta, ida), 2 when none does.
