@@ -1130,7 +1130,7 @@ dr_status dr_render_forward(dr_scene *scene, const dr_render_desc *rd, float *im
         check_cuda(cudaSetDevice(scene->device), "cudaSetDevice");
         scene->last_launches = 0;
         check_cuda(dr_launch_forward(call_scene(scene, rd), rd->width, rd->height, rd->spp, rd->max_bounces, rd->seed, image_dev,
-                                     (cudaStream_t)stream, &scene->last_launches, &scene->timer),
+                                     scene->num_sms, (cudaStream_t)stream, &scene->last_launches, &scene->timer),
                    "forward launch");
         if (scene->timer.failed)
             throw DrError(DR_ERR_CUDA, std::string("kernel ") + scene->timer.failed + " failed: " +

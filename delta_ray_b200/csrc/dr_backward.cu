@@ -31,7 +31,7 @@
 #include "dr_block_grad.cuh"
 
 template <bool kChains, int BMAX>
-__global__ void __launch_bounds__(128, 8) k_backward_paths(const __grid_constant__ DevScene s, int W, int H, int spp, int B, uint64_t seed,
+__global__ void __launch_bounds__(1024, 1) k_backward_paths(const __grid_constant__ DevScene s, int W, int H, int spp, int B, uint64_t seed,
                                                         int lanes_log2, const float *d_image, float *grad, float *img,
                                                         BackwardWorkspace ws, GradCacheCfg cfg) {
     extern __shared__ float sm[];
@@ -45,7 +45,8 @@ __global__ void __launch_bounds__(128, 8) k_backward_paths(const __grid_constant
     float3 acc = f3(0.f);
     int x = active ? (int)(pix % W) : 0, y = active ? (int)(pix / W) : 0;
     float3 dc = active ? f3(d_image[3 * pix], d_image[3 * pix + 1], d_image[3 * pix + 2]) : f3(0.f);
-    // warp-uniform trip count so that the point push can be warp-aggregated
+    // block-uniform trip count: the point push is warp-aggregated, and the barrier
+    // keeps the block's warps in step
     int iters = (spp + G - 1) >> lanes_log2;
     for (int it = 0; it < iters; it++) {
         int si = lane + (it << lanes_log2);
@@ -65,7 +66,7 @@ __global__ void __launch_bounds__(128, 8) k_backward_paths(const __grid_constant
             };
             acc += backward_pixel_sample<kChains, BMAX>(s, x, y, W, H, spp, si, B, seed, dc, bg, push);
         }
-        __syncwarp();
+        __syncthreads();
         unsigned long long slot = warp_reserve(&ws.counters->points, has ? 1 : 0);
         if (has) {
             if (slot < (unsigned long long)ws.cap_points) pr.store(ws.pt + (size_t)slot * DR_PT_WORDS);
@@ -130,10 +131,14 @@ cudaError_t dr_launch_backward_front(const DevScene &s, int W, int H, int spp, i
                                      const float *d_image, float *grad, float *img, long long primary_edge_samples,
                                      int dp_mode, const BackwardWorkspace &ws, const GradCacheCfg &cfg, int num_sms,
                                      cudaStream_t st, int *launches, StageTimer *timer, bool traverse, bool first) {
-    const int bs = 128;
     size_t smem = sizeof(float) * (size_t)(cfg.head + cfg.tail_len);
     int lanes_log2 = path_lanes_log2(spp);
     long long threads = ((long long)W * H) << lanes_log2;
+    // direct lighting is best at 512 (3.6 ms of a 512x512x16-sample soft shadow, 3.7
+    // at 1024, 4.4 at 128), longer paths at 1024 (room of 12 spheres 6.2, 7.1 and
+    // 7.4; 640x480 heightfield 3.7, 3.9 and 4.2); 25,000 samples at 128 (six such
+    // views together 12.9 ms of their streams, 14.6 at 512, 17.1 at 1024)
+    const int bs = path_block(threads, num_sms, B == 1 ? 512 : 1024, 128);
     if (first) timer->begin(st);  // a later view's front stage of a batched call continues the timing
     if (first && (dp_mode != DR_DP_SUM || s.specular_chains)) {
         // LAST: one key per point; SUM with chains: a float4 dp sum per point

@@ -19,15 +19,15 @@ namespace cg = cooperative_groups;
 #ifndef DR_CONNECT_BLOCKS
 #define DR_CONNECT_BLOCKS 8
 #endif
-// and of the line and side-radiance kernels (a sweep at the 640x480
-// heightfield: radiance 3 / 4 / 6 / 8 blocks 264 / 249 / 223 / 234 ms per
-// step)
+// and of the line kernel; threads of the side-radiance kernel's one block per
+// SM, and the blocks per SM that its launch has
 #ifndef DR_LINE_BLOCKS
 #define DR_LINE_BLOCKS 7
 #endif
-#ifndef DR_RADIANCE_BLOCKS
-#define DR_RADIANCE_BLOCKS 6
+#ifndef DR_RADIANCE_THREADS
+#define DR_RADIANCE_THREADS 768
 #endif
+#define DR_RADIANCE_ROUNDS 48
 
 #define DR_ITEM_BUF 24
 // One thread per shading point in [pt_begin, pt_end).  A point's items collect
@@ -435,11 +435,21 @@ __global__ void __launch_bounds__(128, 8) k_edge_line_rays(const __grid_constant
 // multi-bounce shading) in a kernel of its own, [2 h] and [2 h + 1] of
 // ws.side_rad, one lane per side; k_edge_shade then runs without the
 // path-tracing code, whose size made the fused kernel wait on instruction
-// fetches.
-__global__ void __launch_bounds__(128, DR_RADIANCE_BLOCKS) k_edge_radiance(const __grid_constant__ DevScene s, int B,
+// fetches.  One block per SM whose warps start each round of sides together
+// share the instructions they fetch: 640x480 heightfield, 22 M sides, 53.8 ms
+// with six blocks of 128 threads, 38.1 so (768 threads, 80 registers);
+// 160x120 3.45 -> 2.6, room of 12 spheres 4.05 -> 2.4; 384 threads 38.5 and 2.9.
+// Few sides are spread over one block per SM.
+__global__ void __launch_bounds__(DR_RADIANCE_THREADS, 1) k_edge_radiance(const __grid_constant__ DevScene s, int B,
                                                                          uint64_t seed, BackwardWorkspace ws) {
     const long long n = 2 * (long long)min(ws.counters->cands, (unsigned long long)ws.cap_items);
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+    // fewer sides than a round of one block per SM: a part of every block's lanes
+    const int sms = gridDim.x / DR_RADIANCE_ROUNDS;
+    const int width = (int)min((long long)blockDim.x, ((n + sms - 1) / sms + 31) & ~31ll);
+    for (long long q0 = (long long)blockIdx.x * width; q0 < n; q0 += (long long)gridDim.x * width) {
+        __syncthreads();
+        const long long q = q0 + threadIdx.x;
+        if (threadIdx.x >= width || q >= n) continue;
         const int k = (int)(q & 1);
         const int4 hr = ws.hits[q >> 1];
         if (hr.w == 0) continue;
@@ -500,10 +510,13 @@ __global__ void __launch_bounds__(128, 4) k_edge_shade(const __grid_constant__ D
 // code of a forward path), k_primary_grad redraws the sample and turns the
 // color difference into the scene and camera gradients.
 template <int BMAX>
-__global__ void __launch_bounds__(128, 6) k_primary_shade(const __grid_constant__ DevScene s, int B, uint64_t seed, long long i0, long long n,
+__global__ void __launch_bounds__(256, 3) k_primary_shade(const __grid_constant__ DevScene s, int B, uint64_t seed, long long i0, long long n,
                                                        float4 *out) {
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
-        out[k] = primary_shade_item<BMAX>(s, i0 + k, B, seed);
+    for (long long k0 = (long long)blockIdx.x * blockDim.x; k0 < n; k0 += (long long)gridDim.x * blockDim.x) {
+        if (BMAX == 1) __syncthreads();
+        const long long k = k0 + threadIdx.x;
+        if (k < n) out[k] = primary_shade_item<BMAX>(s, i0 + k, B, seed);
+    }
 }
 
 __global__ void __launch_bounds__(128, 8) k_primary_grad(const __grid_constant__ DevScene s, int W, int H, int spp, uint64_t seed,
@@ -638,8 +651,9 @@ cudaError_t dr_launch_edge_traverse(const DevScene &s, uint64_t seed, const Back
         *launches += 1;
         return cudaGetLastError();
     }
-    if (prop) k_edge_traverse<true><<<stage_grid(num_sms), 128, 0, st>>>(s, seed, ws);
-    else k_edge_traverse<false><<<stage_grid(num_sms), 128, 0, st>>>(s, seed, ws);
+    const int grid = (int)std::min<long long>(blocks_for(ws.cap_points, 128), stage_grid_fine(num_sms));
+    if (prop) k_edge_traverse<true><<<grid, 128, 0, st>>>(s, seed, ws);
+    else k_edge_traverse<false><<<grid, 128, 0, st>>>(s, seed, ws);
     timer->mark(st, "k_edge_traverse");
     *launches += 1;
     return cudaGetLastError();
@@ -659,7 +673,7 @@ cudaError_t dr_launch_edge_eval(const DevScene &s, int W, int H, int spp, int B,
     if (s.num_tris <= DR_LINEAR_TRIS) {
         auto line_rays = ext ? (B > 1 ? k_edge_line_rays<true, false> : k_edge_line_rays<true, true>)
                              : (B > 1 ? k_edge_line_rays<false, false> : k_edge_line_rays<false, true>);
-        line_rays<<<grid, 128, 0, st>>>(s, seed, ws);
+        line_rays<<<stage_grid_fine(num_sms), 128, 0, st>>>(s, seed, ws);
         timer->mark(st, "k_edge_line_rays");
         *launches -= 1;
     } else {
@@ -686,7 +700,7 @@ cudaError_t dr_launch_edge_eval(const DevScene &s, int W, int H, int spp, int B,
     }
     const bool pre = B > 1 && ws.side_rad != nullptr;
     if (pre) {
-        k_edge_radiance<<<grid, 128, 0, st>>>(s, B, seed, ws);
+        k_edge_radiance<<<num_sms * DR_RADIANCE_ROUNDS, DR_RADIANCE_THREADS, 0, st>>>(s, B, seed, ws);
         timer->mark(st, "k_edge_radiance");
         *launches += 1;
     }
@@ -709,8 +723,12 @@ cudaError_t dr_launch_primary_edges(const DevScene &s, int W, int H, int spp, in
     auto shade = B == 1 ? k_primary_shade<1> : k_primary_shade<(1 << 30)>;
     for (long long i0 = 0; i0 < n; i0 += cap) {
         long long m = std::min(cap, n - i0);
-        int nb = (int)std::min<long long>(blocks_for(m, bs), (long long)stage_grid(num_sms) * 4);
-        shade<<<nb, bs, 0, st>>>(s, B, seed, i0, m, scratch);
+        // direct lighting: blocks of 256 in step by a barrier per sample (1.63 ->
+        // 1.35 ms for 4 M samples of a soft shadow; longer paths are faster in small
+        // blocks without: 0.54 against 0.58 ms for 0.3 M of a heightfield)
+        const int nb = (int)std::min<long long>(blocks_for(m, bs), (long long)stage_grid_fine(num_sms) * 4);
+        const int sbs = B == 1 ? 256 : 128;
+        shade<<<(nb * bs + sbs - 1) / sbs, sbs, 0, st>>>(s, B, seed, i0, m, scratch);
         timer->mark(st, "k_primary_shade");
         k_primary_grad<<<nb, bs, smem, st>>>(s, W, H, spp, seed, d_image, i0, m, scratch, grad, cfg);
         timer->mark(st, "k_primary_grad");

@@ -79,7 +79,17 @@ cudaError_t dr_launch_eval_math(int fn, const float *x, const float *y, float *o
 cudaError_t dr_launch_trace(const DevScene &s, const float *rays, long long n, int *tri, float *t, cudaStream_t st,
                             int *launches);
 
-cudaError_t dr_launch_forward(const DevScene &s, int W, int H, int spp, int B, uint64_t seed, float *img,
+// Threads of a block for the path kernels, whose code is several times the
+// instruction caches: warps of different blocks are at different places of it
+// and wait for instructions most of the time (17.8 of 31 stall cycles).  One
+// block per SM, its warps in step by a barrier per sample, share what is
+// fetched; with fewer samples than two rounds of such blocks the small block
+// spreads better.
+inline int path_block(long long threads, int num_sms, int large, int small) {
+    return threads >= 2048ll * num_sms ? large : small;
+}
+
+cudaError_t dr_launch_forward(const DevScene &s, int W, int H, int spp, int B, uint64_t seed, float *img, int num_sms,
                               cudaStream_t st, int *launches, StageTimer *timer);
 
 // Backward pass (dr_backward.cu).

@@ -392,13 +392,24 @@ DEV BounceHit sample_bsdf_scene(const DevScene &s, const BSDFSample &bs, float3 
 // shade (pathtrace.h:179-297), forward only.  `rng` is positioned at the first
 // secondary sample; it is taken by value so callers can replay the same draws.
 // BMAX bounds max_bounces at compile time (1: the direct-lighting variant).
-template <int BMAX = 1 << 30>
+// Step says how a path starts a bounce: on its own, or with the paths of its
+// block (every thread calls then, those without a path with alive = false), so
+// that the block's warps fetch the bounce's instructions together.
+struct OwnStep {
+    DEV static bool any(bool alive) { return alive; }
+};
+#ifdef __CUDACC__
+struct BlockStep {
+    __device__ __forceinline__ static bool any(bool alive) { return __syncthreads_or(alive); }
+};
+#endif
+template <int BMAX = 1 << 30, class Step = OwnStep>
 DEV float3 shade(const DevScene &s, float3 wi, int ptri, const SurfacePoint &psp, const LightSample &ls, Rng rng,
-                 int max_bounces, bool include_primary_light) {
+                 int max_bounces, bool include_primary_light, bool alive = true) {
     if (max_bounces > BMAX) max_bounces = BMAX;
     float3 color = f3(0.f);
-    if (ptri < 0) return color;
-    if (include_primary_light) {
+    alive = alive && ptri >= 0;
+    if (alive && include_primary_light) {
         int li = light_of_tri(s, ptri);
         if (li >= 0 && dot(psp.f.n, wi) > 0.f) color += light_intensity(s, li);
     }
@@ -406,17 +417,19 @@ DEV float3 shade(const DevScene &s, float3 wi, int ptri, const SurfacePoint &psp
     float3 cwi = wi;
     int ctri = ptri;
     SurfacePoint csp = psp;
-    for (int b = 0; b < max_bounces; b++) {
+    for (int b = 0; b < max_bounces && Step::any(alive); b++) {
+        if (!alive) continue;
+        alive = false;  // until the bounce is through
         SecondarySample ss = draw_secondary(rng);
         color += thr * nee(s, ls, wi, ctri, csp);
         BounceHit bh = sample_bsdf_scene(s, ss.bsdf, cwi, ctri, csp);
-        if (bh.tri < 0) break;
+        if (bh.tri < 0) continue;
         float3 wo = normalize(bh.sp.p - csp.p);
         int mi = material_of_tri(s, ctri);
         float pdf = bsdf_pdf(s, mi, csp, cwi, wo);
-        if (pdf <= 0.f) break;
+        if (pdf <= 0.f) continue;
         float3 be = bsdf(s, mi, csp, cwi, wo);
-        if (sum(be) <= 0.f) break;
+        if (sum(be) <= 0.f) continue;
         int nli = light_of_tri(s, bh.tri);
         if (nli >= 0 && dot(bh.sp.f.n, -wo) > 0.f) {
             float3 contrib = be * light_intensity(s, nli);
@@ -427,30 +440,34 @@ DEV float3 shade(const DevScene &s, float3 wi, int ptri, const SurfacePoint &psp
         thr = thr * (be / pdf);
         if (b >= 5) {
             float q = fminf(max3(thr), 0.95f);
-            if (ss.rr >= q) break;
+            if (ss.rr >= q) continue;
             thr = thr / q;
         }
         cwi = -wo;
         ctri = bh.tri;
         csp = bh.sp;
+        alive = true;
     }
     return color;
 }
 
 // One pixel sample's radiance contribution (render_sample_fast,
 // delta_ray.cpp:640-692; sub-pixel jitter in [0, 1/spp) as :1236-1237).
-DEV float3 pixel_sample(const DevScene &s, int x, int y, int W, int H, int spp, int si, int B, uint64_t seed) {
+template <class Step = OwnStep>
+DEV float3 pixel_sample(const DevScene &s, int x, int y, int W, int H, int spp, int si, int B, uint64_t seed,
+                        bool alive = true) {
     Rng r;
     r.init(seed, kStreamPixel, ((uint64_t)y * W + x) * spp + si, 0);
     float ux = r.next(), uy = r.next();
     float sub_x = s.full_pixel_jitter ? ux : ux / spp;
     float sub_y = s.full_pixel_jitter ? uy : uy / spp;
     Ray ray = sample_primary(s.cam, float((x + sub_x) / W), float((y + sub_y) / H));
-    if (abs_sum(ray.d) == 0.f) return f3(0.f);
-    Hit h = trace_closest(s, ray.o, ray.d, 1e-3f);
-    if (h.tri < 0) return f3(0.f);
-    SurfacePoint sp = intersect_tri(load_tri(s, h.tri), ray.o, ray.d);
+    Hit h;
+    h.tri = -1;
+    if (alive && abs_sum(ray.d) != 0.f) h = trace_closest(s, ray.o, ray.d, 1e-3f);
+    SurfacePoint sp;
+    if (h.tri >= 0) sp = intersect_tri(load_tri(s, h.tri), ray.o, ray.d);
     LightSample ls = draw_light(r);
-    float3 c = shade(s, -ray.d, h.tri, sp, ls, r, B, true);
+    float3 c = shade<1 << 30, Step>(s, -ray.d, h.tri, sp, ls, r, B, true);
     return c * (1.f / spp);
 }
