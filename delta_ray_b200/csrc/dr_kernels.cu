@@ -208,7 +208,8 @@ cudaError_t dr_launch_trace(const DevScene &s, const float *rays, long long n, i
 // Forward render: one pixel sample per (pixel, lane) and a segmented warp
 // reduction over the 2^lanes_log2 lanes of a pixel.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024, 1) k_render_forward(const __grid_constant__ DevScene s, int W, int H, int spp, int B, uint64_t seed,
+template <class Step>
+__global__ void __launch_bounds__(512, 2) k_render_forward(const __grid_constant__ DevScene s, int W, int H, int spp, int B, uint64_t seed,
                                                         int lanes_log2, float *img) {
     long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     int G = 1 << lanes_log2;
@@ -217,9 +218,9 @@ __global__ void __launch_bounds__(1024, 1) k_render_forward(const __grid_constan
     float3 acc = f3(0.f);
     bool active = pix < (long long)W * H;
     const int x = (int)(pix % W), y = (int)(pix / W);
-    // G divides spp: the trip count is the block's, whose paths go through their
-    // bounces together
-    for (int si = lane; si < spp; si += G) acc += pixel_sample<BlockStep>(s, x, y, W, H, spp, si, B, seed, active);
+    // G divides spp: the trip count is the block's (BlockStep: its paths go
+    // through their bounces together)
+    for (int si = lane; si < spp; si += G) acc += pixel_sample<Step>(s, x, y, W, H, spp, si, B, seed, active);
     for (int off = G >> 1; off >= 1; off >>= 1) {
         acc.x += __shfl_down_sync(0xffffffffu, acc.x, off);
         acc.y += __shfl_down_sync(0xffffffffu, acc.y, off);
@@ -239,10 +240,15 @@ cudaError_t dr_launch_forward(const DevScene &s, int W, int H, int spp, int B, u
         lanes_log2++;
     long long threads = ((long long)W * H) << lanes_log2;
     // 640x480x16-sample heightfield image: 6.2 ms with the large blocks, 6.7 with
-    // blocks of 256 whose paths run on their own
-    const int bs = path_block(threads, num_sms, 1024, 256);
+    // blocks of 256 whose paths run on their own; a room of 8 spheres at 529x377x2
+    // samples 0.95 and 1.14.  Scenes traced without a tree and direct lighting wait
+    // more at the barriers than they gain (triangle at 640x480x8 samples 0.150
+    // against 0.115 ms, soft shadow 0.425 and 0.408), as do smaller images (row
+    // of 100x80 to 190x180 pixels: 5 to 15 %)
+    const int bs = s.num_tris > DR_LINEAR_TRIS && B > 1 ? path_block(threads, num_sms, 512, 256) : 256;
+    auto kernel = bs == 256 ? k_render_forward<OwnStep> : k_render_forward<BlockStep>;
     timer->begin(st);
-    k_render_forward<<<blocks_for(threads, bs), bs, 0, st>>>(s, W, H, spp, B, seed, lanes_log2, img);
+    kernel<<<blocks_for(threads, bs), bs, 0, st>>>(s, W, H, spp, B, seed, lanes_log2, img);
     timer->mark(st, "k_render_forward");
     *launches += 1;
     return cudaGetLastError();
