@@ -394,12 +394,16 @@ DEV BounceHit sample_bsdf_scene(const DevScene &s, const BSDFSample &bs, float3 
 // BMAX bounds max_bounces at compile time (1: the direct-lighting variant).
 // Step says how a path starts a bounce: on its own, or with the paths of its
 // block (every thread calls then, those without a path with alive = false), so
-// that the block's warps fetch the bounce's instructions together.
+// that the block's warps fetch the bounce's instructions together.  A path on
+// its own leaves the loop where it ends (soft shadow image, 640x480x8 samples:
+// 0.764 ms, 0.773 with the flag tested at the next bounce).
 struct OwnStep {
-    DEV static bool any(bool alive) { return alive; }
+    static constexpr bool kOwn = true;
+    DEV static bool any(bool) { return true; }
 };
 #ifdef __CUDACC__
 struct BlockStep {
+    static constexpr bool kOwn = false;
     __device__ __forceinline__ static bool any(bool alive) { return __syncthreads_or(alive); }
 };
 #endif
@@ -417,19 +421,31 @@ DEV float3 shade(const DevScene &s, float3 wi, int ptri, const SurfacePoint &psp
     float3 cwi = wi;
     int ctri = ptri;
     SurfacePoint csp = psp;
+    if (Step::kOwn && !alive) return color;
     for (int b = 0; b < max_bounces && Step::any(alive); b++) {
-        if (!alive) continue;
-        alive = false;  // until the bounce is through
+        if (!Step::kOwn) {
+            if (!alive) continue;
+            alive = false;  // until the bounce is through
+        }
         SecondarySample ss = draw_secondary(rng);
         color += thr * nee(s, ls, wi, ctri, csp);
         BounceHit bh = sample_bsdf_scene(s, ss.bsdf, cwi, ctri, csp);
-        if (bh.tri < 0) continue;
+        if (bh.tri < 0) {
+            if (Step::kOwn) break;
+            continue;
+        }
         float3 wo = normalize(bh.sp.p - csp.p);
         int mi = material_of_tri(s, ctri);
         float pdf = bsdf_pdf(s, mi, csp, cwi, wo);
-        if (pdf <= 0.f) continue;
+        if (pdf <= 0.f) {
+            if (Step::kOwn) break;
+            continue;
+        }
         float3 be = bsdf(s, mi, csp, cwi, wo);
-        if (sum(be) <= 0.f) continue;
+        if (sum(be) <= 0.f) {
+            if (Step::kOwn) break;
+            continue;
+        }
         int nli = light_of_tri(s, bh.tri);
         if (nli >= 0 && dot(bh.sp.f.n, -wo) > 0.f) {
             float3 contrib = be * light_intensity(s, nli);
@@ -440,13 +456,16 @@ DEV float3 shade(const DevScene &s, float3 wi, int ptri, const SurfacePoint &psp
         thr = thr * (be / pdf);
         if (b >= 5) {
             float q = fminf(max3(thr), 0.95f);
-            if (ss.rr >= q) continue;
+            if (ss.rr >= q) {
+                if (Step::kOwn) break;
+                continue;
+            }
             thr = thr / q;
         }
         cwi = -wo;
         ctri = bh.tri;
         csp = bh.sp;
-        alive = true;
+        if (!Step::kOwn) alive = true;
     }
     return color;
 }
