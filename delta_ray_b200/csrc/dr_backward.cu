@@ -3,13 +3,17 @@
 //   k_backward_paths   one thread per (pixel, lane): path adjoint of the
 //                      pixel's samples, image, and the shading-point records
 //   k_edge_traverse    one thread per shading point: edge-tree traversal,
-//                      appends (point, edge, weight) items
-//   k_edge_line        one thread per item: the line sample on the edge
+//                      appends (point, edge, weight) items (small trees;
+//                      larger ones: k_walk_ctx and k_edge_walk, a warp walking
+//                      a few points' subtrees together)
+//   k_line_ctx, k_edge_line  the points' line set-ups; a warp's run of items in
+//                      phases: the line sample on each edge
 //   k_edge_connect     surviving line samples fetched one per lane: the
 //                      connectivity of the two straddling rays (the edge's
 //                      faces, bounded occlusion walks)
 //   k_edge_pairs       candidates fetched one per lane: the other side's
 //                      closest hit and the tests on both hits
+//   k_edge_radiance    one thread per side of a kept sample: its radiance (B > 1)
 //   k_edge_shade       one thread per kept sample: shading of both sides,
 //                      dv0/dv1 scatter and dp
 //   k_dp_propagate     one thread per point: the point's dp through its
