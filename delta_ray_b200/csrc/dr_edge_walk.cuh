@@ -26,25 +26,8 @@
 // ran alone); with one step for every node that splits or draws 83 and 5.9.
 #pragma once
 
-// Pending nodes per warp, by class: 2 the all walk's nodes that split (bound
-// above 1, or around the point), whose children's bounds only meet thresholds
-// and whose cone tests decide nothing (k_edge_walk's fast step; three in four
-// nodes of a glossy heightfield); of the others, 1 the all walk's off the cone
-// walk's path, 0 the rest, which take the cone tests.
-//
-// While all stacks have room for a step's children the classes are stepped as
-// they fill.  Without that room (or room to hand the nodes on) no node goes to
-// class 2 any more (`two`): a child then stays in its parent's class or goes to
-// class 1, and a step takes only as many nodes as leave
-// DR_WALK_RESERVE slots of its class free, and at least one.  Taking one at a
-// time needs one slot per tree level (trees are split at the median: at most
-// 28 levels, node ids having 27 bits), so the reserve always suffices; steps
-// of classes 0 and 2 also add up to 32 nodes to the classes below, which are
-// drained first.
-#define DR_WALK_N0 128
-#define DR_WALK_N1 128
-#define DR_WALK_N2 224
-#define DR_WALK_RESERVE 32
+#include "dr_walk_rules.cuh"
+
 #define DR_WALK_POINTS 4  // points of a batch, at most
 #define DR_WALK_ITEMS 128
 #ifndef DR_WALK_BLOCKS
@@ -133,7 +116,7 @@ template <bool PROP> struct WalkWarp {
     static constexpr int kCtx = PROP ? 44 : 32;  // words of a context
     float4 ctx[DR_WALK_POINTS][kCtx / 4 + 1];    // one float4 of padding: slots start in different banks
     uint2 st[DR_WALK_N0 + DR_WALK_N1 + DR_WALK_N2];  // pending nodes, class after class: code, apmf
-    float c[DR_WALK_N0 + DR_WALK_N2];                // cpmf of classes 0 and 2 (class 1's is 0)
+    float c[DR_WALK_N0 + DR_WALK_N2];                // cpmf of classes 0 and 2 (class 1's is 0 or NaN)
     float l[PROP ? DR_WALK_N0 + DR_WALK_N1 + DR_WALK_N2 : 1];  // lpmf
     uint2 leaf[64];        // edge or node | slot << 27 | mode << 30 | many << 31, weight
     uint2 item[DR_WALK_ITEMS];  // edge | slot << 27 | mode << 30, weight
@@ -188,14 +171,15 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
         // a node to its class's stack, every lane's at once
         const int b1 = DR_WALK_N0, b2 = DR_WALK_N0 + DR_WALK_N1;  // where classes 1 and 2 begin
         const auto push_nodes = [&](bool node, unsigned code, float cp, float ap, float lp) {
-            const bool all_walk = (code >> 30) & 1;
-            const bool to2 = node && two && all_walk && (code >> 31), to0 = node && !to2 && (!all_walk || cp != 0.f);
-            const unsigned m0 = __ballot_sync(full, to0), m2 = __ballot_sync(full, to2),
-                           m1 = __ballot_sync(full, node && !to0 && !to2);
+            const int cls = walk_class(code, cp, two);
+            const bool to0 = node && cls == 0, to1 = node && cls == 1, to2 = node && cls == 2;
+            const unsigned m0 = __ballot_sync(full, to0), m1 = __ballot_sync(full, to1), m2 = __ballot_sync(full, to2);
             if (node) {
                 const int at = to0 ? n0 + __popc(m0 & below)
                                    : (to2 ? b2 + n2 + __popc(m2 & below) : b1 + n1 + __popc(m1 & below));
-                sh.st[at] = make_uint2(code, __float_as_uint(ap));
+                // class 1 keeps no cp: the mode's bit, set in all of its nodes,
+                // is cleared where it is NaN
+                sh.st[at] = make_uint2(to1 && cp != 0.f ? code & ~(1u << 30) : code, __float_as_uint(ap));
                 if (to0) sh.c[at] = cp;
                 else if (to2) sh.c[at - DR_WALK_N1] = cp;
                 if constexpr (PROP) sh.l[at] = lp;
@@ -203,6 +187,15 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
             n0 += __popc(m0);
             n1 += __popc(m1);
             n2 += __popc(m2);
+        };
+        // the pending node at `at`: its cp, and its code with the mode's bit
+        const auto node_at = [&](int at, unsigned &code, float &cp) {
+            if (at >= b1 && at < b2) {
+                cp = (code >> 30) & 1 ? 0.f : __int_as_float(0x7fc00000);
+                code |= 1u << 30;
+            } else {
+                cp = sh.c[at < b1 ? at : at - DR_WALK_N1];
+            }
         };
         if (in) {  // the handed-on nodes
             const bool have = lane < pk->count;
@@ -313,9 +306,7 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
             }
         };
         for (int steps = 0; n0 + n1 + n2 > 0; steps++) {
-            const bool room = n0 <= DR_WALK_N0 - DR_WALK_RESERVE - 32 && n1 <= DR_WALK_N1 - DR_WALK_RESERVE - 32 &&
-                              n2 <= DR_WALK_N2 - 32;
-            if (two && (!room || (steps >= DR_WALK_STEPS && n0 + n1 + n2 >= DR_WALK_HAND))) {
+            if (two && (!walk_room(n0, n1, n2) || (steps >= DR_WALK_STEPS && n0 + n1 + n2 >= DR_WALK_HAND))) {
                 // the pending nodes to the next round: packet q of np takes
                 // every np-th, so that large and small subtrees spread
                 const int n = n0 + n1 + n2, np = (n + 31) >> 5;
@@ -329,10 +320,10 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
                     const int i = q + lane * np;
                     if (fits && i < n) {
                         const int at = i < n0 ? i : (i < n0 + n1 ? b1 + i - n0 : b2 + i - n0 - n1);
-                        const uint2 e = sh.st[at];
-                        float l = 0.f;
+                        uint2 e = sh.st[at];
+                        float l = 0.f, cp;
                         if constexpr (PROP) l = sh.l[at];
-                        const float cp = at < b1 ? sh.c[at] : (at >= b2 ? sh.c[at - DR_WALK_N1] : 0.f);
+                        node_at(at, e.x, cp);
                         o->e[lane] = make_uint4(e.x, e.y, __float_as_uint(cp), __float_as_uint(l));
                     }
                     // no room for all: the packets there is room for are left
@@ -346,28 +337,9 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
                 if (fits) break;
                 two = false;
             }
-            // Up to 16 nodes: of one class where a class fills the step, else of
-            // all (which only the general step takes).  k0, k1, k2: the nodes
-            // taken of each class.
-            int k0 = 0, k1 = 0, k2 = 0;
-            const bool fast = two && n2 >= 16;
-            if (fast) {
-                k2 = 16;
-            } else if (!two) {  // short of room: class 1 first, then 0, which add to none but themselves and 1
-                if (n1 >= 16) k1 = min(16, max(1, DR_WALK_N1 - n1 - DR_WALK_RESERVE));
-                else if (n0 >= 16) k0 = min(16, max(1, DR_WALK_N0 - n0 - DR_WALK_RESERVE));
-                else if (n2 > 0) k2 = min(16, n2);
-                else if (n0 > 0) k0 = min(min(16, n0), max(1, DR_WALK_N0 - n0 - DR_WALK_RESERVE));
-                else k1 = n1;
-            } else if (n1 >= 16) {
-                k1 = 16;
-            } else if (n0 >= 16) {
-                k0 = 16;
-            } else {
-                k2 = n2;
-                k1 = min(n1, 16 - k2);
-                k0 = min(n0, 16 - k2 - k1);
-            }
+            const WalkTake take = walk_take(n0, n1, n2, two);
+            const int k0 = take.k0, k1 = take.k1, k2 = take.k2;
+            const bool fast = take.fast;
             const int k = k0 + k1 + k2;
             const int j = lane >> 1;
             const bool right = lane & 1, act = j < k;
@@ -378,7 +350,7 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
                 const uint2 e = sh.st[at];
                 code = e.x;
                 apmf = __uint_as_float(e.y);
-                cpmf = at < b1 ? sh.c[at] : (at >= b2 ? sh.c[at - DR_WALK_N1] : 0.f);
+                node_at(at, code, cpmf);
                 if constexpr (PROP) lpmf = sh.l[at];
             }
             n0 -= k0;

@@ -49,6 +49,7 @@ def load():
         L.hh_trace_pairs.argtypes = [C.POINTER(_abi.dr_scene_desc), C.c_void_p, C.c_int, C.c_void_p]
         L.hh_trace_before.argtypes = [C.POINTER(_abi.dr_scene_desc), C.c_void_p, C.c_void_p, C.c_void_p, C.c_int,
                                       C.c_void_p]
+        L.hh_walk_stacks.argtypes = [C.c_int] * 7 + [C.c_void_p]
         _lib = L
     return _lib
 
@@ -164,3 +165,12 @@ def silhouette(lo, hi, axis, angle, p):
     out = np.zeros((n, 2), np.int32)
     L.hh_silhouette(*[a.ctypes.data for a in arrs], n, out.ctypes.data)
     return out[:, 0].astype(bool), out[:, 1].astype(bool)
+
+
+def walk_stacks(seed, trials, levels, child, split, off, nan):
+    """The most pending nodes the warp walk's three stacks hold over made-up
+    walks that cannot hand nodes on (hh_walk_stacks), and the steps they took
+    without room."""
+    out = np.zeros(4, np.int64)
+    load().hh_walk_stacks(seed, trials, levels, child, split, off, nan, out.ctypes.data)
+    return out[:3], int(out[3])

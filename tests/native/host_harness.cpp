@@ -25,6 +25,7 @@ static int g_ckpt = 0;
 
 #include "../../delta_ray_b200/csrc/dr_backward.cuh"
 #include "../../delta_ray_b200/csrc/dr_bvh.cuh"
+#include "../../delta_ray_b200/csrc/dr_walk_rules.cuh"
 #include "../../delta_ray_b200/csrc/dr_host_scene.h"
 
 namespace {
@@ -402,6 +403,55 @@ void hh_trace_before(const dr_scene_desc *desc, const float *rays, const float *
         const float3 o = f3(r[0], r[1], r[2]), d = f3(r[3], r[4], r[5]);
         out[2 * i] = trace_before_bvh(b.ds.bvh_nodes, b.ds.bvh_tris, b.ds.bvh_root, o, d, 1e-3f, ta[i], ida[i]);
         out[2 * i + 1] = trace_before_wide(wide.data(), b.ds.bvh_tris, b.ds.bvh_root, o, d, 1e-3f, ta[i], ida[i]);
+    }
+}
+
+// The warp walk's stacks under its own rules (dr_walk_rules.cuh) over `trials`
+// made-up walks whose nodes have up to two children `levels` levels deep, with
+// shares and splits drawn to fill the stacks (percentages: `child` a child is
+// walked, `split` it splits the all walk, `off` it leaves the cone walk's path,
+// `nan` its share is undefined), and whose nodes cannot be handed on.
+// out: the most entries each class held, then the steps taken without room.
+void hh_walk_stacks(int seed, int trials, int levels, int child, int split, int off, int nan, long long *out) {
+    struct Node { unsigned code; float cp; int level; };
+    uint64_t state = 0x9E3779B97F4A7C15ull * (uint64_t)(seed + 1);
+    const auto chance = [&](int percent) {
+        state ^= state << 13, state ^= state >> 7, state ^= state << 17;
+        return (int)((state >> 20) % 100) < percent;
+    };
+    for (int i = 0; i < 4; i++) out[i] = 0;
+    for (int t = 0; t < trials; t++) {
+        std::vector<Node> st[3];
+        bool two = true;
+        const auto push = [&](Node n) { st[walk_class(n.code, n.cp, two)].push_back(n); };
+        for (int b = 0; b < 4; b++)  // both walks of a batch of points, as k_edge_walk begins them
+            for (unsigned mode = 0; mode < 2; mode++) st[0].push_back(Node{mode << 30, 0.5f, 0});
+        for (long long steps = 0; steps < 20000; steps++) {
+            const int n[3] = {(int)st[0].size(), (int)st[1].size(), (int)st[2].size()};
+            if (n[0] + n[1] + n[2] == 0) break;
+            if (two && !walk_room(n[0], n[1], n[2])) two = false;
+            out[3] += !two;
+            const WalkTake take = walk_take(n[0], n[1], n[2], two);
+            const int k[3] = {take.k0, take.k1, take.k2};
+            std::vector<Node> taken;
+            for (int c = 0; c < 3; c++)
+                for (int i = 0; i < k[c]; i++) {
+                    taken.push_back(st[c].back());
+                    st[c].pop_back();
+                }
+            for (const Node &p : taken)
+                for (int c = 0; c < 2; c++) {
+                    if (p.level + 1 >= levels || !chance(child)) continue;
+                    Node n{p.code & (1u << 30), p.cp, p.level + 1};
+                    if (chance(split)) n.code |= 1u << 31;
+                    if (!take.fast) {  // a node that splits passes its share on
+                        if (chance(off)) n.cp = p.cp * 0.f;
+                        else if (chance(nan)) n.cp = p.cp * NAN;
+                    }
+                    push(n);
+                }
+            for (int c = 0; c < 3; c++) out[c] = std::max(out[c], (long long)st[c].size());
+        }
     }
 }
 
