@@ -43,6 +43,7 @@ def lib():
     L.dr_eval_math.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p]
     L.dr_scene_last_work.argtypes = [C.c_void_p, C.c_void_p, C.c_int]
     L.dr_set_item_queue_limit.argtypes = [C.c_int64]
+    L.dr_scene_set_walk_packets.argtypes = [C.c_void_p, C.c_int64]
     L.dr_scene_edge_data.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_int64, C.POINTER(C.c_int64),
                                      C.POINTER(C.c_float)]
     L.dr_scene_set_profiling.argtypes = [C.c_void_p, C.c_int]
@@ -65,7 +66,8 @@ def lib():
                  "dr_render_forward", "dr_render_backward", "dr_scene_last_launch_count", "dr_trace_rays",
                  "dr_scene_set_profiling", "dr_scene_last_timings", "dr_scene_last_counts", "dr_eval_math",
                  "dr_scene_edge_data", "dr_scene_last_work",
-                 "dr_set_item_queue_limit", "dr_scene_get_tuning", "dr_scene_set_tuning", "dr_scene_autotune"):
+                 "dr_set_item_queue_limit", "dr_scene_set_walk_packets", "dr_scene_get_tuning", "dr_scene_set_tuning",
+                 "dr_scene_autotune"):
         getattr(L, name).restype = C.c_int
     if L.dr_abi_version() != 2:
         raise ImportError("libdr_b200.so has an unexpected ABI version")

@@ -253,6 +253,7 @@ struct dr_scene {
     }
     int last_launches = 0;
     dr_tuning tune{64, 3, 0, 0, 0};  // dr_scene_set_tuning
+    long long walk_packets = 0;      // dr_scene_set_walk_packets (0: the default)
 };
 
 namespace {
@@ -718,6 +719,7 @@ std::pair<long long, long long> run_backward(dr_scene *scene, const dr_render_de
         work[4] += (long long)(c.tasks + c.handed_total);
         work[5] += (long long)(ds.split_traversal ? c.items_expand : c.items);
         work[8] += (long long)c.cands;
+        for (int r = 0; r < DR_WALK_ROUNDS; r++) work[9] += (long long)c.walk_n[r];
     };
     // edges per bucket of points [p0, p0 + np) from ws.pt_items
     auto read_buckets_at = [&](long long p0, long long np, std::vector<unsigned long long> &out) {
@@ -1208,6 +1210,7 @@ void backward_on_queues(dr_scene *scene, const dr_render_desc *rd, const DevScen
             q.walk_ctx.reserve(sizeof(float4) * DR_CTX_F4 * cap_points);
             ws.walk_ctx = q.walk_ctx.as<float4>();
             ws.cap_packets = std::min(kMaxPackets, std::max(kMinPackets, 4 * cap_points));
+            if (scene->walk_packets > 0) ws.cap_packets = std::min(ws.cap_packets, scene->walk_packets);
             q.packets.reserve((size_t)DR_WALK_PACKET_BYTES * 2 * ws.cap_packets);
             ws.packets = q.packets.p;
         }
@@ -1739,6 +1742,14 @@ dr_status dr_scene_last_work(const dr_scene *scene, int64_t *counts, int n) {
     return guard([&]() {
         if (!scene || !counts || n < 0) throw DrError(DR_ERR_INVALID_ARGUMENT, "NULL argument");
         for (int i = 0; i < n && i < 10; i++) counts[i] = scene->last_work[i];
+    });
+}
+
+dr_status dr_scene_set_walk_packets(dr_scene *scene, int64_t packets) {
+    return guard([&]() {
+        if (!scene) throw DrError(DR_ERR_INVALID_ARGUMENT, "scene is NULL");
+        if (packets < 0) throw DrError(DR_ERR_INVALID_ARGUMENT, "negative packet bound");
+        scene->walk_packets = (long long)packets;
     });
 }
 

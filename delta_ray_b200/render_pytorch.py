@@ -274,17 +274,23 @@ class Scene:
         first-stage items,
         node visits of the point walks and of the large trees' walks,
         candidates of the ray stage (samples that passed its connectivity
-        test), and 0 (reserved)."""
+        test), and packets of pending nodes the large trees' walks had to hand
+        on between rounds."""
         w = (C.c_int64 * 10)()
         _lib.check(_lib.lib().dr_scene_last_work(self.handle, w, 10))
         keys = ("points", "items", "survivors", "shaded", "tasks", "items_first_stage", "visits_walk",
-                "visits_tasks", "candidates", "spilled")
+                "visits_tasks", "candidates", "packets")
         return dict(zip(keys, (int(x) for x in w)))
 
     def last_counts(self):
         p, it = C.c_int64(), C.c_int64()
         _lib.check(_lib.lib().dr_scene_last_counts(self.handle, C.byref(p), C.byref(it)))
         return p.value, it.value
+
+    def set_walk_packets(self, packets=0):
+        """Bounds the packets of pending nodes a round of the large trees'
+        walks can hand on (dr_scene_set_walk_packets; 0: the default)."""
+        _lib.check(_lib.lib().dr_scene_set_walk_packets(self.handle, int(packets)))
 
     def launch_count(self):
         n = C.c_int()

@@ -386,9 +386,17 @@ DR_API dr_status dr_scene_edge_data(const dr_scene *scene, int what, void *out_h
  * [5] edges sampled by the first stage (all, when the traversal runs in one
  * stage), [6] edge-tree nodes visited by the point walks, [7] nodes
  * visited by the walks of large trees, [8] line samples whose connectivity test
- * passed (candidates of the ray stage), [9] 0 (reserved).  Up to n of
- * them are written. */
+ * passed (candidates of the ray stage), [9] packets of pending nodes that the
+ * walks of large trees had to hand on between their rounds, those that found
+ * no room included (dr_scene_set_walk_packets).  Up to n of them are written. */
 DR_API dr_status dr_scene_last_work(const dr_scene *scene, int64_t *counts, int n);
+
+/* Tooling: bound on the packets of pending nodes (32 each) that a round of the
+ * scene's large-tree walks can hand on; 0 restores the default (4 per shading
+ * point, between 16,384 and 1,048,576).  A warp that finds no room walks its
+ * nodes itself, so no bound changes which edges are sampled.  A negative bound
+ * fails with DR_ERR_INVALID_ARGUMENT. */
+DR_API dr_status dr_scene_set_walk_packets(dr_scene *scene, int64_t packets);
 
 /* Kernel launch count of the last render call on this scene (for tooling). */
 DR_API dr_status dr_scene_last_launch_count(const dr_scene *scene, int *count);
