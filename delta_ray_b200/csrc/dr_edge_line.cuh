@@ -207,7 +207,8 @@ __global__ void __launch_bounds__(128, DR_LINE_BLOCKS) k_edge_line(const __grid_
                         }
                     }
                 }
-                const unsigned mask = __ballot_sync(full, ok);  // every lane has read its line
+                const unsigned mask = __ballot_sync(full, ok);
+                __syncwarp();  // every lane has read its line (a vote orders no memory)
                 if (ok) {
                     const int k = kept + __popc(mask & below);
                     t.f[0][k] = __int_as_float(i);
