@@ -717,7 +717,7 @@ std::pair<long long, long long> run_backward(dr_scene *scene, const dr_render_de
         work[2] += (long long)c.survivors;
         work[3] += (long long)c.hits;
         work[4] += (long long)(c.tasks + c.handed_total);
-        work[5] += (long long)(ds.split_traversal ? c.items_expand : c.items);
+        work[5] += (long long)(ds.split_traversal && ws.tasks ? c.items_expand : c.items);  // two stages: depth first
         work[8] += (long long)c.cands;
         for (int r = 0; r < DR_WALK_ROUNDS; r++) work[9] += (long long)c.walk_n[r];
     };
