@@ -33,6 +33,6 @@ def test_first_stage_edges(grid, stages):
             w = sc.last_work()
             assert w["items_first_stage"] == w["items"] > 0
         else:
-            assert 0 < w["items_first_stage"] < w["items"]
+            assert w["items_first_stage"] < w["items"]  # none where every leaf lies deeper than its 8 levels
     finally:
         sc.close()
