@@ -1,6 +1,13 @@
 // CUDA kernels of the renderer: LBVH build and the forward pixel-sample kernel.
 // The per-sample logic lives in the dr_*.cuh headers; kernels here only map
 // threads to work and reduce results.
+//
+// pow, exp and log inlined: a forward path has three call sites, and the calls
+// cost it more than the instructions they share (the backward kernels have
+// them out of line; images of 0.02 to 1.2 ms, calls against inlined: soft shadow
+// at 512x512x16 samples 0.606 and 0.598 ms, mirror hall at 512x384x4 1.048 and
+// 0.962, heightfields at 640x480x4 1.224 and 1.188).
+#define DR_MATH_INLINE
 #include "dr_bvh.cuh"
 #include "dr_kernels.h"
 #include "dr_shading.cuh"
@@ -220,7 +227,8 @@ __global__ void __launch_bounds__(512, 2) k_render_forward(const __grid_constant
     const int x = (int)(pix % W), y = (int)(pix / W);
     // G divides spp: the trip count is the block's (BlockStep: its paths go
     // through their bounces together)
-    for (int si = lane; si < spp; si += G) acc += pixel_sample<Step>(s, x, y, W, H, spp, si, B, seed, active);
+    if (active || !Step::kOwn)
+        for (int si = lane; si < spp; si += G) acc += pixel_sample<Step>(s, x, y, W, H, spp, si, B, seed, active);
     for (int off = G >> 1; off >= 1; off >>= 1) {
         acc.x += __shfl_down_sync(0xffffffffu, acc.x, off);
         acc.y += __shfl_down_sync(0xffffffffu, acc.y, off);
@@ -239,12 +247,14 @@ cudaError_t dr_launch_forward(const DevScene &s, int W, int H, int spp, int B, u
     while ((1 << (lanes_log2 + 1)) <= spp && (1 << (lanes_log2 + 1)) <= 32 && spp % (1 << (lanes_log2 + 1)) == 0)
         lanes_log2++;
     long long threads = ((long long)W * H) << lanes_log2;
-    // 640x480x16-sample heightfield image: 6.2 ms with the large blocks, 6.7 with
-    // blocks of 256 whose paths run on their own; a room of 8 spheres at 529x377x2
-    // samples 0.95 and 1.14.  Scenes traced without a tree and direct lighting wait
-    // more at the barriers than they gain (triangle at 640x480x8 samples 0.150
-    // against 0.115 ms, soft shadow 0.425 and 0.408), as do smaller images (row
-    // of 100x80 to 190x180 pixels: 5 to 15 %)
+    // Large blocks in step against blocks of 256 whose paths run on their own:
+    // 640x480x16-sample heightfield image 5.56 and 6.35 ms, a room of 8 spheres at
+    // 529x377x2 samples, three bounces, 0.83 and 0.96.  Small images wait more at
+    // the barriers than they gain (100x80 heightfield 0.104 against 0.090 ms), and
+    // scenes traced without a tree and direct lighting go both ways (triangle at
+    // 640x480x8 samples 0.137 against 0.105, soft shadow 0.416 and 0.391, but a
+    // mirror hall at 512x384x4 0.82 and 0.96, 640x480x4 heightfields with direct
+    // lighting 0.68 and 0.77): they keep the small blocks.
     const int bs = s.num_tris > DR_LINEAR_TRIS && B > 1 ? path_block(threads, num_sms, 512, 256) : 256;
     auto kernel = bs == 256 ? k_render_forward<OwnStep> : k_render_forward<BlockStep>;
     timer->begin(st);

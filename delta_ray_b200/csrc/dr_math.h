@@ -32,7 +32,11 @@
 
 #if defined(__CUDACC__)
 #define DRM_FN __host__ __device__ __forceinline__
+#ifdef DR_MATH_INLINE
+#define DRM_OUT DRM_FN
+#else
 #define DRM_OUT static __host__ __device__ __noinline__
+#endif
 #else
 #define DRM_FN inline
 #define DRM_OUT inline

@@ -413,6 +413,7 @@ DEV float3 shade(const DevScene &s, float3 wi, int ptri, const SurfacePoint &psp
     if (max_bounces > BMAX) max_bounces = BMAX;
     float3 color = f3(0.f);
     alive = alive && ptri >= 0;
+    if (Step::kOwn && !alive) return color;
     if (alive && include_primary_light) {
         int li = light_of_tri(s, ptri);
         if (li >= 0 && dot(psp.f.n, wi) > 0.f) color += light_intensity(s, li);
@@ -421,7 +422,6 @@ DEV float3 shade(const DevScene &s, float3 wi, int ptri, const SurfacePoint &psp
     float3 cwi = wi;
     int ctri = ptri;
     SurfacePoint csp = psp;
-    if (Step::kOwn && !alive) return color;
     for (int b = 0; b < max_bounces && Step::any(alive); b++) {
         if (!Step::kOwn) {
             if (!alive) continue;
@@ -484,6 +484,7 @@ DEV float3 pixel_sample(const DevScene &s, int x, int y, int W, int H, int spp, 
     Hit h;
     h.tri = -1;
     if (alive && abs_sum(ray.d) != 0.f) h = trace_closest(s, ray.o, ray.d, 1e-3f);
+    if (Step::kOwn && h.tri < 0) return f3(0.f);
     SurfacePoint sp;
     if (h.tri >= 0) sp = intersect_tri(load_tri(s, h.tri), ray.o, ray.d);
     LightSample ls = draw_light(r);
