@@ -116,7 +116,7 @@ template <bool PROP> struct WalkWarp {
     static constexpr int kCtx = PROP ? 44 : 32;  // words of a context
     float4 ctx[DR_WALK_POINTS][kCtx / 4 + 1];    // one float4 of padding: slots start in different banks
     uint2 st[DR_WALK_N0 + DR_WALK_N1 + DR_WALK_N2];  // pending nodes, class after class: code, apmf
-    float c[DR_WALK_N0 + DR_WALK_N2];                // cpmf of classes 0 and 2 (class 1's is 0 or NaN)
+    float c[DR_WALK_N0 + DR_WALK_N2];                // cpmf of classes 0 and 2 (class 1's is 0)
     float l[PROP ? DR_WALK_N0 + DR_WALK_N1 + DR_WALK_N2 : 1];  // lpmf
     uint2 leaf[64];        // edge or node | slot << 27 | mode << 30 | many << 31, weight
     uint2 item[DR_WALK_ITEMS];  // edge | slot << 27 | mode << 30, weight
@@ -177,9 +177,7 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
             if (node) {
                 const int at = to0 ? n0 + __popc(m0 & below)
                                    : (to2 ? b2 + n2 + __popc(m2 & below) : b1 + n1 + __popc(m1 & below));
-                // class 1 keeps no cp: the mode's bit, set in all of its nodes,
-                // is cleared where it is NaN
-                sh.st[at] = make_uint2(to1 && cp != 0.f ? code & ~(1u << 30) : code, __float_as_uint(ap));
+                sh.st[at] = make_uint2(code, __float_as_uint(ap));
                 if (to0) sh.c[at] = cp;
                 else if (to2) sh.c[at - DR_WALK_N1] = cp;
                 if constexpr (PROP) sh.l[at] = lp;
@@ -188,15 +186,8 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
             n1 += __popc(m1);
             n2 += __popc(m2);
         };
-        // the pending node at `at`: its cp, and its code with the mode's bit
-        const auto node_at = [&](int at, unsigned &code, float &cp) {
-            if (at >= b1 && at < b2) {
-                cp = (code >> 30) & 1 ? 0.f : __int_as_float(0x7fc00000);
-                code |= 1u << 30;
-            } else {
-                cp = sh.c[at < b1 ? at : at - DR_WALK_N1];
-            }
-        };
+        // the cone-walk share of the pending node at `at`
+        const auto share_at = [&](int at) { return at < b1 ? sh.c[at] : (at >= b2 ? sh.c[at - DR_WALK_N1] : 0.f); };
         if (in) {  // the handed-on nodes
             const bool have = lane < pk->count;
             uint4 e = make_uint4(0, 0, 0, 0);
@@ -320,11 +311,10 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
                     const int i = q + lane * np;
                     if (fits && i < n) {
                         const int at = i < n0 ? i : (i < n0 + n1 ? b1 + i - n0 : b2 + i - n0 - n1);
-                        uint2 e = sh.st[at];
-                        float l = 0.f, cp;
+                        const uint2 e = sh.st[at];
+                        float l = 0.f;
                         if constexpr (PROP) l = sh.l[at];
-                        node_at(at, e.x, cp);
-                        o->e[lane] = make_uint4(e.x, e.y, __float_as_uint(cp), __float_as_uint(l));
+                        o->e[lane] = make_uint4(e.x, e.y, __float_as_uint(share_at(at)), __float_as_uint(l));
                     }
                     // no room for all: the packets there is room for are left
                     // empty and the warp walks on itself
@@ -350,7 +340,7 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
                 const uint2 e = sh.st[at];
                 code = e.x;
                 apmf = __uint_as_float(e.y);
-                node_at(at, code, cpmf);
+                cpmf = share_at(at);
                 if constexpr (PROP) lpmf = sh.l[at];
             }
             n0 -= k0;
@@ -456,6 +446,7 @@ __global__ void __launch_bounds__(128, DR_WALK_BLOCKS) k_edge_walk(const __grid_
             }
             ccpmf = (right ? sh2.prc : sh2.plc) * cpmf;
             capmf = (right ? sh2.pra : sh2.pla) * apmf;
+            walk_undefined(!cone_mode, ccpmf, capmf);
             clpmf = pl * lpmf;
             }
             const bool leaf = push && (child & DR_CHILD_LEAF);

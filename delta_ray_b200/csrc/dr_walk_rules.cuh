@@ -10,10 +10,12 @@
 // heightfield); of the others, 1 the all walk's off the cone walk's path, 0 the
 // rest, which take the cone tests.
 //
-// Off the path a node's cone-walk share cp is 0, or NaN (0 times an undefined
-// share, below a node with an infinite importance: its box is centred on the
-// point).  Both go to class 1, whose children then all go to class 1 (or 2):
-// class 1 never adds to class 0.
+// Off the path a node's cone-walk share cp is 0, and its children's are 0 too
+// unless their own share is undefined (0 times NaN, below a node with an
+// infinite bound).  The all walk's weight of an edge, ap / (cp^2 + ap^2), is NaN
+// where either share is, and nothing else reads them there, so such a child
+// takes its undefined share as ap and 0 as cp (walk_undefined): class 1 never
+// adds to class 0.
 //
 // While all stacks have room for a step's children (walk_room) the classes are
 // stepped as they fill.  Without that room (or room to hand the nodes on) no
@@ -35,12 +37,20 @@ static_assert(DR_WALK_RESERVE >= DR_WALK_LEVELS, "one node at a time needs a slo
 static_assert(DR_WALK_N0 >= 2 * (DR_WALK_RESERVE + 32) && DR_WALK_N1 >= 2 * (DR_WALK_RESERVE + 32) && DR_WALK_N2 >= 64,
               "room for a step's children above the reserve");
 
+// An all-walk child whose cone-walk share is undefined (see above).
+DEV void walk_undefined(bool all_walk, float &cp, float &ap) {
+    if (all_walk && cp != cp) {
+        ap = cp;
+        cp = 0.f;
+    }
+}
+
 // The class of a node with code `code` (mode << 30, all-split << 31) and
 // cone-walk share cp.
 DEV int walk_class(unsigned code, float cp, bool two) {
     const bool all_walk = (code >> 30) & 1;
     if (two && all_walk && (code >> 31)) return 2;
-    return all_walk && !(fabsf(cp) > 0.f) ? 1 : 0;
+    return all_walk && cp == 0.f ? 1 : 0;
 }
 
 // Whether every stack has room for a step's children with the reserve left.

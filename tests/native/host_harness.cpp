@@ -447,6 +447,8 @@ void hh_walk_stacks(int seed, int trials, int levels, int child, int split, int 
                     if (!take.fast) {  // a node that splits passes its share on
                         if (chance(off)) n.cp = p.cp * 0.f;
                         else if (chance(nan)) n.cp = p.cp * NAN;
+                        float ap = 1.f;
+                        walk_undefined((n.code >> 30) & 1, n.cp, ap);
                     }
                     push(n);
                 }
