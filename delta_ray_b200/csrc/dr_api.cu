@@ -1780,6 +1780,8 @@ size_t dr_last_error(char *buf, size_t len) {
 namespace {
 constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;  // per device
 constexpr long long kNoAllocMaxSamples = 65536;            // width * height * spp
+constexpr size_t kNoAllocCounterBytes = 256;               // the counters, ahead of the point records
+static_assert(sizeof(BackwardCounters) <= kNoAllocCounterBytes, "the counters would run into the point records");
 }  // namespace
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
@@ -1828,7 +1830,7 @@ dr_status dr_render_backward_noalloc(dr_scene *scene, const dr_render_desc *rd, 
             long long fit = (long long)(kNoAllocScratchBytes / 2 / (sizeof(float) * DR_PT_FLOATS + DR_PT_LAST_BYTES));
             cap_points = std::max(npix, std::min(want, fit));
         }
-        size_t off = 256;
+        size_t off = kNoAllocCounterBytes;
         BackwardWorkspace ws{};
         ws.counters = (BackwardCounters *)base;
         ws.pt = (float *)(base + off);
