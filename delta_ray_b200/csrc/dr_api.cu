@@ -373,7 +373,8 @@ void upload_scene(dr_scene *sc, cudaStream_t st, bool refit = false) {
     if (n > 0 && !linear) {
         // the build's working arrays stay with the scene: an update with new
         // vertex positions refits the same tree (closest hits do not depend on
-        // the tree's shape, ties going to the lower triangle id)
+        // the tree's shape, ties going to the lower triangle id, but for rays along
+        // shared edges: trace_before_wide)
         size_t sb = dr_lbvh_scratch_bytes(n);
         if (refit && sc->bvh_built_tris == n && sc->bvh_scratch.bytes >= sb) {
             check_cuda(dr_refit_lbvh(vtx, tri, n, bvh_nodes, bvh_tris, sc->bvh_scratch.p, sc->bvh_scratch.bytes, st,

@@ -514,59 +514,6 @@ DEV bool leaf_entered(float4 a, float4 b, float4 c, float3 o, float3 inv, float 
                      tmax) >= 0.f;
 }
 
-// The walk of trace_before_bvh as a resumable state: begin() sets it up,
-// step() takes one node (a box pair or a leaf) and returns 0 while the walk
-// goes on, 1 when a triangle hits ahead of (ta, ida), 2 when none does.
-// Kernels that interleave many such walks step every walking lane together.
-struct BeforeWalk {
-    float3 o, d, inv;
-    float tnear, ta;
-    int ida, sp, node;
-    int stack[DR_WIDE_STACK];
-    DEV void begin(int root, float3 o_, float3 d_, float tnear_, float ta_, int ida_) {
-        o = o_;
-        d = d_;
-        inv = f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
-        tnear = tnear_;
-        ta = ta_;
-        ida = ida_;
-        sp = 0;
-        node = root;
-    }
-    // wide (may be null): the 4-wide form of the tree, walked in its place
-    DEV int step(const float4 *DR_RESTRICT nodes, const float4 *DR_RESTRICT wide, const float4 *DR_RESTRICT tris) {
-        if (node < 0) {
-            const int leaf = ~node;
-            float4 a = dr_ldg(tris + 3 * leaf), b = dr_ldg(tris + 3 * leaf + 1), c = dr_ldg(tris + 3 * leaf + 2);
-            float t;
-            if (hit_triangle(a, b, c, o, d, t) && t > tnear && (t < ta || (t == ta && dr_f2i(a.w) < ida))) return 1;
-            if (sp == 0) return 2;
-            node = stack[--sp];
-            return 0;
-        }
-        if (wide) return wide_next(wide_kids(wide + (size_t)DR_WIDE_F4 * node, o, inv, ta), stack, sp, node) ? 0 : 2;
-        const float4 *n = nodes + 4 * node;
-        float4 n0 = dr_ldg(n), n1 = dr_ldg(n + 1), n2 = dr_ldg(n + 2), n3 = dr_ldg(n + 3);
-        float e0 = box_entry(n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, o, inv, ta);
-        float e1 = box_entry(n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, o, inv, ta);
-        int c0 = dr_f2i(n3.x), c1 = dr_f2i(n3.y);
-        bool h0 = e0 >= 0.f, h1 = e1 >= 0.f;
-        if (h0 && h1) {
-            int nearc = e0 <= e1 ? c0 : c1, farc = e0 <= e1 ? c1 : c0;
-            if (sp < DR_STACK) stack[sp++] = farc;
-            node = nearc;
-        } else if (h0) {
-            node = c0;
-        } else if (h1) {
-            node = c1;
-        } else {
-            if (sp == 0) return 2;
-            node = stack[--sp];
-        }
-        return 0;
-    }
-};
-
 // Whether a triangle hits ahead of (ta, ida) under the closest-hit rule: at t
 // on (tnear, ta), or at ta with a smaller id.  Boxes are culled at ta (the
 // widened test keeps every box holding such a hit), nearer child first.
@@ -610,14 +557,18 @@ DEV_NOINLINE bool trace_before_bvh(const float4 *DR_RESTRICT nodes, const float4
 }
 
 // ---------------------------------------------------------------------------
-// Walks of the 4-wide form of the LBVH (DevScene::bvh_wide), taken by the
-// warp-stepped occlusion walks (BeforeWalk) and by trace_before; closest and
-// any hits walk the binary nodes (see trace_closest).  Each step tests
-// a node's (up to) four children, the binary walk's two levels at once, in
-// the same boxes, and goes on with the nearest child entered, the others
-// stacked nearest on top.  The hits are those of the binary walks: a box is
-// culled only beyond the best hit so far, and the closest-hit rule (smallest
-// t, ties to the smaller triangle id) does not depend on the order.
+// The bounded walk over the 4-wide form of the LBVH (DevScene::bvh_wide), which
+// trace_before takes; the ray stage's kernel steps the same nodes with
+// fast_kids, and closest and any hits walk the binary nodes (measured faster
+// there).  Each step tests a node's (up to) four children, the binary walk's two
+// levels at once, in the same boxes, and goes on with the nearest child entered,
+// the others stacked nearest on top.  The answer is the binary walk's: both cull
+// boxes at the same fixed distance, so they test the same triangles whatever
+// the order.  (A closest-hit walk culls at its best hit so far.  Its hits are the
+// same in any order but for rays along shared edges, where a triangle's
+// rounded distance falls short of its box by more than the box test allows:
+// walked far child first, 13 of 300,000 rays aimed at a heightfield's vertices
+// end on the neighbouring triangle.)
 DEV_NOINLINE bool trace_before_wide(const float4 *DR_RESTRICT wide, const float4 *DR_RESTRICT tris, int root,
                                     float3 o, float3 d, float tnear, float ta, int ida) {
     const float3 inv = f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
