@@ -237,13 +237,17 @@ DEV BoundCtx bound_ctx(float3 wi, const SurfacePoint &sp, float dl, float sl, fl
 // evaluation: the silhouette filter's sine, cosine and reciprocal square root
 // (absolute errors below 1e-6 on its arguments) and the bound filter's log2
 // and exp2 (a few ulps).  The filters only ever decide with margins well above
-// those errors.
+// those errors.  DR_FILT_ERR: the CPU tests give the values errors as large as
+// the device's.
 #ifdef DR_HOST_BUILD
+#ifndef DR_FILT_ERR
+#define DR_FILT_ERR(x) (x)
+#endif
 HD float filt_sin(float x) { return std::sin(x); }
 HD float filt_cos(float x) { return std::cos(x); }
-HD float filt_rsqrt(float x) { return 1.f / std::sqrt(x); }
-HD float filt_log2(float x) { return std::log2(x); }
-HD float filt_exp2(float x) { return std::exp2(x); }
+HD float filt_rsqrt(float x) { return DR_FILT_ERR(1.f / std::sqrt(x)); }
+HD float filt_log2(float x) { return DR_FILT_ERR(std::log2(x)); }
+HD float filt_exp2(float x) { return DR_FILT_ERR(std::exp2(x)); }
 #else
 DEV float filt_sin(float x) { return __sinf(x); }
 DEV float filt_cos(float x) { return __cosf(x); }
@@ -253,7 +257,7 @@ DEV float filt_exp2(float x) { return exp2f(x); }
 #endif
 // a / b to a few ulps (b > 0 and not huge)
 #ifdef DR_HOST_BUILD
-HD float filt_div(float a, float b) { return a / b; }
+HD float filt_div(float a, float b) { return DR_FILT_ERR(a / b); }
 #else
 DEV float filt_div(float a, float b) { return __fdividef(a, b); }
 #endif
@@ -1215,15 +1219,18 @@ DEV void hit_faces_pair(const EdgeRec *rec, float3 o, float3 dr, float3 dl, floa
 // its faces, decided before the sample is drawn: the rays lean out of the
 // plane through p and the edge by delta = 1e-3 |sample_p| (edge_side_dirs), so
 // a face must reach that far out of the plane to be hit, and small faces far
-// away do not.  With n the plane's unit normal, X a hit and D the faces' least
-// distance from p, |X . n| >= D (delta - eta) / (1 + delta), eta the angle by
-// which the sample's direction itself may leave the plane (rounding of the
-// lobe's transform m: 1e-6 |m| |x| for points x of the line), while no point
-// of a face has a larger |X . n| than its corner opposite the edge.  Answers
-// true only with a tenth to spare, and 1e-6 |a|^3 / |(v0 - p) x (v1 - p)| for
-// the rounding of n: the hit test's own error is far smaller there (its
-// coordinate of the opposite corner has a relative error of a few
-// 2^-24 / delta, delta - eta being at least 1e-5).
+// away do not.  With n the plane's unit normal and X a hit, relative to p: X's
+// part in the plane is at least D long, as X lies on a face, within
+// max(|v1 - v0|, |a - v0|) of v0, and the projection to the plane, which holds
+// v0, brings it no farther; along n the ray gains delta - eta per length in the
+// plane, so |X . n| >= D (delta - eta).  eta is the angle by which the sample's
+// direction itself may leave the plane (rounding of the lobe's transform m:
+// 1e-6 |m| |x| for points x of the line), and delta at least 1e-3 times the
+// edge's least distance (`near`).  No point of a face has a larger |X . n|
+// than its corner opposite the edge.  Answers true only with a tenth to spare,
+// and 1e-6 |a|^3 / |(v0 - p) x (v1 - p)| for the rounding of n: the hit test's
+// own error is far smaller there (its coordinate of the opposite corner has a
+// relative error of a few 2^-24 / delta, delta - eta being at least 1e-5).
 // L: a bound on the lengths of the line's points x in the lobe's space.
 DEV bool faces_out_of_reach(const EdgeRec *rec, float3 v0, float3 v1, float3 p, const M3 &m, float L) {
     const float4 qa = dr_ldg(&rec->r[2]), qb = dr_ldg(&rec->r[3]);

@@ -50,6 +50,9 @@ def load():
         L.hh_trace_before.argtypes = [C.POINTER(_abi.dr_scene_desc), C.c_void_p, C.c_void_p, C.c_void_p, C.c_int,
                                       C.c_void_p]
         L.hh_walk_stacks.argtypes = [C.c_int] * 7 + [C.c_void_p]
+        L.hh_trace_before_fast.argtypes = L.hh_trace_before.argtypes
+        L.hh_bound_side.argtypes = [C.c_void_p] * 8 + [C.c_longlong, C.c_int, C.c_void_p]
+        L.hh_faces_reach.argtypes = [C.c_void_p] * 7 + [C.c_longlong, C.c_void_p, C.c_int, C.c_void_p]
         _lib = L
     return _lib
 
@@ -174,3 +177,37 @@ def walk_stacks(seed, trials, levels, child, split, off, nan):
     out = np.zeros(4, np.int64)
     load().hh_walk_stacks(seed, trials, levels, child, split, off, nan, out.ctypes.data)
     return out[:3], int(out[3])
+
+
+def trace_before_fast(wl, rays, ta, ida):
+    """Whether a triangle hits ahead of (ta, ida) for rays [n, 6], as the
+    connectivity kernel's box tests decide it and through the binary walk: [n, 2] int."""
+    from delta_ray_b200 import _abi
+    L = load()
+    cam, mats, shps, lts = _abi.scene_dicts(wl.camera, wl.materials, wl.shapes, wl.lights)
+    sd = _abi.SceneDesc.from_scene(cam, mats, shps, lts, torch.device("cpu"))
+    rays, ta = np.ascontiguousarray(rays, np.float32), np.ascontiguousarray(ta, np.float32)
+    ida = np.ascontiguousarray(ida, np.int32)
+    out = np.zeros((rays.shape[0], 2), np.int32)
+    L.hh_trace_before_fast(C.byref(sd.desc), rays.ctypes.data, ta.ctypes.data, ida.ctypes.data, rays.shape[0],
+                           out.ctypes.data)
+    return out
+
+
+def bound_side(lo, hi, p, normal, wi, dl, sl, rough, ulps):
+    """Blinn-Phong bounds of boxes (hh_bound_side): decided [n] bool, the side
+    bound, its relative margin and the exact bound (float32 [n] each)."""
+    arrs = [np.ascontiguousarray(a, np.float32) for a in (lo, hi, p, normal, wi, dl, sl, rough)]
+    out = np.zeros((len(arrs[5]), 4), np.float32)
+    load().hh_bound_side(*[a.ctypes.data for a in arrs], len(out), int(ulps), out.ctypes.data)
+    return out[:, 0] != 0, out[:, 1], out[:, 2], out[:, 3]
+
+
+def faces_reach(v0, v1, a, b, p, minv, m, u):
+    """Edges' faces against their line samples' side rays (hh_faces_reach): out
+    of reach [n] bool, and the draws whose rays hit a face [n] (-1: no line)."""
+    arrs = [np.ascontiguousarray(x, np.float32) for x in (v0, v1, a, b, p, minv, m)]
+    u = np.ascontiguousarray(u, np.float32)
+    out = np.zeros((len(arrs[0]), 2), np.int32)
+    load().hh_faces_reach(*[x.ctypes.data for x in arrs], len(out), u.ctypes.data, len(u), out.ctypes.data)
+    return out[:, 0] != 0, out[:, 1]

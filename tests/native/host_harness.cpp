@@ -23,6 +23,18 @@ static int g_split = 0;
 // form, segments of k bounces (0: the per-bounce records)
 static int g_ckpt = 0;
 
+// relative error of up to g_filt_ulps ulps, drawn per value, of the node
+// filters' fast functions (0: none), as the device's have (hh_bound_side)
+static int g_filt_ulps = 0;
+static unsigned g_filt_state = 1;
+static float filt_err(float x) {
+    if (g_filt_ulps == 0) return x;
+    g_filt_state = g_filt_state * 1664525u + 1013904223u;
+    const int r = (int)(g_filt_state >> 16) % (2 * g_filt_ulps + 1) - g_filt_ulps;
+    return x * (1.f + (float)r * 1.1920929e-7f);
+}
+#define DR_FILT_ERR(x) filt_err(x)
+
 #include "../../delta_ray_b200/csrc/dr_backward.cuh"
 #include "../../delta_ray_b200/csrc/dr_bvh.cuh"
 #include "../../delta_ray_b200/csrc/dr_walk_rules.cuh"
@@ -453,6 +465,113 @@ void hh_walk_stacks(int seed, int trials, int levels, int child, int split, int 
                     push(n);
                 }
             for (int c = 0; c < 3; c++) out[c] = std::max(out[c], (long long)st[c].size());
+        }
+    }
+}
+
+// The same test as k_edge_connect decides it: boxes with fused multiply-adds
+// (fast_kids), a blocker only if its own box is entered (leaf_entered), inner
+// nodes before leaves.  out[2i] its answer, out[2i + 1] the binary walk's.
+void hh_trace_before_fast(const dr_scene_desc *desc, const float *rays, const float *ta, const int *ida, int n,
+                          int *out) {
+    HostSceneBundle b;
+    make_scene(desc, b);
+    const int ni = b.ds.num_tris - 1;
+    std::vector<float4> wide((size_t)DR_WIDE_F4 * std::max(ni, 1));
+    for (int p = 0; p < ni; p++) widen_node(b.ds.bvh_nodes, p, wide.data() + (size_t)DR_WIDE_F4 * p);
+    for (int i = 0; i < n; i++) {
+        const float *r = rays + 6 * i;
+        const float3 o = f3(r[0], r[1], r[2]), d = f3(r[3], r[4], r[5]);
+        const float3 inv = f3(safe_inv(d.x), safe_inv(d.y), safe_inv(d.z));
+        const FastRay ray = fast_ray(o, inv);
+        std::vector<int> nodes{b.ds.bvh_root}, leaves;
+        while (!nodes.empty()) {
+            const int node = nodes.back();
+            nodes.pop_back();
+            if (node < 0) {
+                leaves.push_back(~node);
+                continue;
+            }
+            const FastKids kids = fast_kids(wide.data() + (size_t)DR_WIDE_F4 * node, ray, ta[i]);
+            if (!kids.any) continue;
+            nodes.push_back(kids.c[0]);
+            for (int c = 1; c < 4; c++)
+                if (kids.hit[c]) nodes.push_back(kids.c[c]);
+        }
+        out[2 * i] = 0;
+        for (int leaf : leaves) {
+            const float4 *q = b.ds.bvh_tris + 3 * leaf;
+            float t;
+            if (hit_triangle(q[0], q[1], q[2], o, d, t) && t > 1e-3f &&
+                (t < ta[i] || (t == ta[i] && dr_f2i(q[0].w) < ida[i])) &&
+                leaf_entered(q[0], q[1], q[2], o, inv, ta[i]))
+                out[2 * i] = 1;
+        }
+        out[2 * i + 1] = trace_before_bvh(b.ds.bvh_nodes, b.ds.bvh_tris, b.ds.bvh_root, o, d, 1e-3f, ta[i], ida[i]);
+    }
+}
+
+// The Blinn-Phong bound of n boxes, exact and by its sides (bsdf_bound_side,
+// its fast functions off by up to `ulps` ulps): box lo[3k], hi[3k] seen from
+// p[3k] with normal nrm[3k] and direction wi[3k], reflectances dl[k], sl[k],
+// roughness[k].  out[4k]: decided, the side bound, its relative margin, exact.
+void hh_bound_side(const float *lo, const float *hi, const float *p, const float *nrm, const float *wi, const float *dl,
+                   const float *sl, const float *rough, long long n, int ulps, float *out) {
+    const auto at = [](const float *a, long long k) { return f3(a[3 * k], a[3 * k + 1], a[3 * k + 2]); };
+    for (long long k = 0; k < n; k++) {
+        SurfacePoint sp{};
+        sp.p = at(p, k);
+        sp.f.n = at(nrm, k);
+        const BoundCtx c = bound_ctx(at(wi, k), sp, dl[k], sl[k], rough[k], 0);
+        float bound = 0.f, fm = 0.f;
+        g_filt_ulps = ulps;
+        const bool decided = bsdf_bound_side(at(lo, k), at(hi, k), c, bound, fm);
+        g_filt_ulps = 0;
+        out[4 * k] = decided;
+        out[4 * k + 1] = bound;
+        out[4 * k + 2] = fm;
+        out[4 * k + 3] = bsdf_bound_box(at(lo, k), at(hi, k), c, nullptr);
+    }
+}
+
+// Line samples of n edges v0, v1 with faces' opposite vertices a, b seen from
+// p (3 floats each) through lobe transforms minv, m (9 floats each), at the
+// draws u[nu]: out[2k] whether the faces are out of the side rays' reach
+// (faces_out_of_reach), out[2k + 1] how many of the draws' side rays hit one
+// (-1: the edge gives no line).
+void hh_faces_reach(const float *v0, const float *v1, const float *a, const float *b, const float *p, const float *minv,
+                    const float *m, long long n, const float *u, int nu, int *out) {
+    const auto at = [](const float *x, long long k) { return f3(x[3 * k], x[3 * k + 1], x[3 * k + 2]); };
+    for (long long k = 0; k < n; k++) {
+        const float3 e0 = at(v0, k), e1 = at(v1, k), q[2] = {at(a, k), at(b, k)}, o = at(p, k);
+        EdgeRec rec{};
+        rec.r[0].x = e0.x, rec.r[0].y = e0.y, rec.r[0].z = e0.z;
+        rec.r[1].x = e1.x, rec.r[1].y = e1.y, rec.r[1].z = e1.z;
+        rec.r[2].x = q[0].x, rec.r[2].y = q[0].y, rec.r[2].z = q[0].z;
+        rec.r[3].x = q[1].x, rec.r[3].y = q[1].y, rec.r[3].z = q[1].z;
+        rec.r[4].w = dr_i2f(36 | (36 << 6));  // corners v0, v1, opposite of both faces
+        rec.r[5].x = dr_i2f(0), rec.r[5].y = dr_i2f(1);
+        M3 mi, mm;
+        for (int i = 0; i < 9; i++) mi.m[i] = minv[9 * k + i], mm.m[i] = m[9 * k + i];
+        out[2 * k] = 0, out[2 * k + 1] = -1;
+        float3 ca, cb;
+        LineState ln;
+        if (!line_clip(mi, e0, e1, o, ca, cb)) continue;
+        out[2 * k] = faces_out_of_reach(&rec, e0, e1, o, mm, fmaxf(abs_sum(ca), abs_sum(cb)));
+        if (!line_begin(ca, cb, ln)) continue;
+        out[2 * k + 1] = 0;
+        for (int j = 0; j < nu; j++) {
+            LineSolve sv;
+            sv.begin(ln);
+            while (!sv.step(ln, u[j])) {
+            }
+            EdgeLine el;
+            el.sample_p = mul(mm, ln.vo + sv.l * ln.wt);
+            float3 sdir, rdir, ldir;
+            edge_side_dirs(el, e0, e1, o, sdir, rdir, ldir);
+            Hit hr, hl;
+            hit_faces_pair(&rec, o, rdir, ldir, 1e-3f, hr, hl);
+            out[2 * k + 1] += hr.tri >= 0 || hl.tri >= 0;
         }
     }
 }
