@@ -189,9 +189,9 @@ def kernel_bytes(kernel, wl, work):
     n = W * H * spp
     P, I = work["points"], work["items"]
     rays_path = 1 + 2 * B  # upper bound: camera ray, then a shadow and a BSDF ray per bounce
-    # an edge sample's shading: two shadow rays to the emitters, plus the
-    # multi-bounce paths of both sides when B > 1 (1 + 2 (B - 1) rays each)
-    shade_rays = 2 + (2 * (1 + 2 * (B - 1)) if B > 1 else 0)
+    # an edge sample's shading: two shadow rays to the emitters; with B > 1 the
+    # multi-bounce paths of both sides (1 + 2 (B - 1) rays each) run before it
+    side_rays = 2 * (1 + 2 * (B - 1)) if B > 1 else 0
     if kernel == "k_render_forward":
         return n * (rays_path * br + B * SHADE_BYTES) + W * H * 12
     if kernel == "k_backward_paths":
@@ -226,11 +226,24 @@ def kernel_bytes(kernel, wl, work):
         return work.get("candidates", 0) * (16 + 32 + br + 16)
     if kernel == "k_edge_line_rays":
         return I * (20 + POINT_BYTES + 36 + 28) + work["survivors"] * 2 * br + work["shaded"] * 48
-    if kernel == "k_edge_shade":  # records in, shading rays and vertices, dp out, vertex gradient adds
-        return work["shaded"] * (48 + POINT_BYTES + shade_rays * br + 2 * SHADE_BYTES + 12 + 2 * 12)
+    if kernel == "k_edge_radiance":  # records in, both sides' rays and vertices, their radiance out
+        return work["shaded"] * (48 + POINT_BYTES + side_rays * br + 2 * (B - 1) * SHADE_BYTES + 32)
+    if kernel == "k_edge_shade":  # records in, shadow rays and vertices, dp out, vertex gradient adds
+        return work["shaded"] * (48 + POINT_BYTES + (32 if B > 1 else 0) + 2 * br + 2 * SHADE_BYTES + 12 + 2 * 12)
     if kernel == "k_dp_propagate":
         return P * (POINT_BYTES + 36 + 12 * 3)
     return 0
+
+
+def memory_roofline(ms, model_bytes, dram_bytes, peak):
+    """A kernel's memory rate against the measured copy's `peak` (GB/s): from
+    its profiled DRAM bytes, or (dram_bytes None) from the byte model's, which
+    count every node and record a walk reads, most of them cache hits.  A kernel
+    whose DRAM rate is below half of the peak is not bound by it."""
+    rate = (model_bytes if dram_bytes is None else dram_bytes) / (ms / 1e3) / 1e9 if ms > 0 else 0.0
+    on_chip = dram_bytes is not None and rate < 0.5 * peak
+    return {"bound": "on-chip (instructions, L1, L2)" if on_chip else "hbm", "achieved": rate, "frac": rate / peak,
+            "bytes": "model" if dram_bytes is None else "DRAM (profiled)"}
 
 
 def load_peaks():
@@ -619,19 +632,18 @@ def run_b200(args):
     e2e_s = max_over_ranks((time.perf_counter() - t0) / e2e_steps)
     e2e_value = world * samples / e2e_s
 
-    # roofline of the dominant kernel (the longest one of a step, its
-    # launches summed)
+    # roofline of the dominant kernel (the longest one of a step, its launches
+    # summed)
     peak, peak_kind = load_peaks()
     dom = max(stages, key=lambda s: s[1]) if stages else ("", 0.0)
     dom_bytes = kernel_bytes(dom[0], wl, work)
-    achieved = dom_bytes / (dom[1] / 1e3) / 1e9 if dom[1] > 0 else 0.0
     prof = load_profile(dom[0])
     traffic = None
     if prof:  # DRAM bytes of the captured launch, scaled to this launch's units
         units = work["items"] if dom[0].startswith("k_edge") else samples
         traffic = int(prof["dram_bytes"] * units / max(1, prof["units"]))
-    roofline = {"bound": "hbm", "kernel": dom[0], "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": achieved / peak, "peak_kind": peak_kind, "traffic": traffic,
+    roofline = {"kernel": dom[0], **memory_roofline(dom[1], dom_bytes, traffic, peak), "peak": peak, "unit": "GB/s",
+                "peak_kind": peak_kind, "traffic": traffic,
                 "algorithmic_bytes_per_step": dom_bytes,
                 "l2": ({"hit_rate_pct": prof["l2_hit_pct"], "throughput_pct_of_peak": prof["l2_throughput_pct"],
                         "source": prof["source"]} if prof else None),
