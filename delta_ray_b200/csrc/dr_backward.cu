@@ -138,10 +138,14 @@ cudaError_t dr_launch_backward_front(const DevScene &s, int W, int H, int spp, i
     size_t smem = sizeof(float) * (size_t)(cfg.head + cfg.tail_len);
     int lanes_log2 = path_lanes_log2(spp);
     long long threads = ((long long)W * H) << lanes_log2;
-    // direct lighting is best at 512 (3.6 ms of a 512x512x16-sample soft shadow, 3.7
-    // at 1024, 4.4 at 128), longer paths at 1024 (room of 12 spheres 6.2, 7.1 and
-    // 7.4; 640x480 heightfield 3.7, 3.9 and 4.2); 25,000 samples at 128 (six such
-    // views together 12.9 ms of their streams, 14.6 at 512, 17.1 at 1024)
+    // Against blocks of 128, 512 and 1024 take: with more than direct lighting a room
+    // of 12 spheres 7.4 ms, 7.1 and 6.2, 640x480 heightfields 4.2, 3.9 and 3.7.  With
+    // direct lighting both are faster than 128: the soft shadow, which has the most
+    // samples, is best at 512 (4.6, 3.6 and 3.7), meshes and glossy scenes at 1024 (a
+    // room of 8 spheres at 640x480x2 2.33, 2.02 and 1.76, glossy shadow 512x512x4
+    // 2.24, 1.52 and 1.29, 64x64-vertex heightfield 320x240x8 3.69, 3.48 and 3.46).
+    // 25,000 samples at 128 (six such views together 12.9 ms of their streams, 14.6 at
+    // 512, 17.1 at 1024)
     const int bs = path_block(threads, num_sms, B == 1 ? 512 : 1024, 128);
     if (first) timer->begin(st);  // a later view's front stage of a batched call continues the timing
     if (first && (dp_mode != DR_DP_SUM || s.specular_chains)) {

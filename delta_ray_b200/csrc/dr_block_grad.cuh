@@ -43,7 +43,10 @@ struct BlockGradWarp : BlockGrad {
 // adding to one shared entry one after another made a launch of 25,000 samples
 // in a room of 12 spheres take 3.2 ms, 2.1 with this; where most adds are a
 // full warp's to one entry the plain form is the faster one (k_primary_grad on
-// the soft shadow 1.37 against 1.76 ms).
+// the soft shadow 1.37 against 1.76 ms).  In mirror scenes of a few materials, whose
+// groups are nearly the whole of the active lanes, the rounds cost more than
+// they save (k_backward_paths, 300x200x4 samples, three bounces: 3.1 ms, 2.8
+// with the plain form; 64x48x2, five bounces: 0.71 and 0.54).
 struct BlockGradGroups : BlockGrad {
     __device__ __forceinline__ void add(int i, float v) {
         const unsigned mask = __activemask();

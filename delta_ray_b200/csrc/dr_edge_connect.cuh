@@ -14,20 +14,20 @@
 // took one as soon as they were idle, left the warp split into groups issuing
 // on their own: 5.1 and 3.8 of 32 lanes active.)
 //
-// What bounds it: L1 throughput (each walking lane reads its own 128-byte
-// node) and issue.  So a lane first tests the last triangle it found in the
-// way: samples follow each other by edge, and at the 130,054-triangle
-// heightfield a blocker of the sample before blocks about half of the occluded
-// right rays, the right ray's four in five of the left rays beside it, and a
-// walk saved is about 45 nodes.  Any triangle that the walk would test and
-// that blocks gives its answer (leaf_entered).  The boxes are tested with fused
-// multiply-adds, which enter a few more than the walk's own test would.  The
-// walk's stack lies in shared memory, a
-// column per lane (in local memory it took as much of the L1's throughput as
-// the nodes).  Measured there: 99 -> 69.5 ms at 640x480, 1 spp (120 M samples),
-// 6.3 -> 4.5 at 160x120, 19 of 32 lanes active (14.7 before).  Dropped: lanes
-// taking runs of 2, 4 or 8 samples (7.1 ms with 8: neighbouring samples no
-// longer share their nodes' cache lines across the warp), 6 and 7 blocks per SM.
+// What bounds it: L1 throughput (77 % of its peak: each walking lane reads its
+// own 128-byte node) and issue (73 % of the slots).  So a lane first tests the
+// last triangle it found in the way: samples follow each other by edge, and at
+// the 130,054-triangle heightfield a blocker of the sample before blocks about
+// half of the occluded right rays, the right ray's four in five of the left rays
+// beside it, and a walk saved is about 45 nodes.  Any triangle that the walk
+// would test and that blocks gives its answer (leaf_entered).  The boxes are
+// tested with fused multiply-adds, which enter a few more than the walk's own
+// test would.  The walk's stack lies in shared memory, a column per lane (in
+// local memory it took as much of the L1's throughput as the nodes).  Measured
+// there: 99 -> 69.5 ms at 640x480, 1 spp (120 M samples), 6.3 -> 4.5 at 160x120,
+// 17.1 of 32 lanes active (14.7 before).  Dropped: lanes taking runs of 2, 4 or 8
+// samples (7.1 ms with 8: neighbouring samples no longer share their nodes' cache
+// lines across the warp), 6 and 7 blocks per SM.
 #define DR_CONNECT_STACK 20  // deeper entries (up to DR_WIDE_STACK) go to local memory
 __global__ void __launch_bounds__(128, DR_CONNECT_BLOCKS) k_edge_connect(const __grid_constant__ DevScene s, BackwardWorkspace ws) {
     __shared__ int stack[DR_CONNECT_STACK][128];

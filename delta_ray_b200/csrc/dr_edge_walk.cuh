@@ -2,16 +2,19 @@
 // batch of points with its pending nodes in shared memory.  Included by
 // dr_edge_kernels.cu.
 //
-// What bounds it: instruction issue and fetch (a node decision is 300 to 450
-// instructions per child, most of them the BSDF bound's).  Two lanes share a
-// node, one per child, so that a lane evaluates one bound, reads its child
-// with two 16-byte loads next to its partner's, and exchanges importances and
-// tests with one shuffle each: 16 nodes a step.  The nodes come off stacks by
-// class, so that the lanes of a step run one path: the nodes that split the all
-// walk (three in four of a glossy heightfield's) need no draw, no cone tests
-// and only a bound's sides of 0 and 1.  The points' contexts, the stacks, the
-// reached leaves and the sampled edges stay in shared memory: a node costs no
-// global traffic but its own record, and the items leave in runs of
+// What bounds it: instruction fetch and latency.  A node decision is 300 to 450
+// instructions per child, most of them the BSDF bound's; at the 160x120
+// heightfield below issue slots are 55 % busy with 37 % of the warps resident
+// (shared memory holds them to 7 blocks per SM), 22.3 of 32 lanes active, and
+// warps wait for instructions first (4.4 cycles per issue, then 2.3 for fixed
+// latencies).  Two lanes share a node, one per child, so that a lane evaluates
+// one bound, reads its child with two 16-byte loads next to its partner's, and
+// exchanges importances and tests with one shuffle each: 16 nodes a step.  The
+// nodes come off stacks by class, so that the lanes of a step run one path: the
+// nodes that split the all walk (three in four of a glossy heightfield's) need no
+// draw, no cone tests and only a bound's sides of 0 and 1.  The points' contexts,
+// the stacks, the reached leaves and the sampled edges stay in shared memory: a
+// node costs no global traffic but its own record, and the items leave in runs of
 // consecutive slots, each point's together (the line and ray kernels then read
 // one point's data and neighbouring edges from a warp's lanes).
 //
@@ -21,7 +24,7 @@
 // the 130,054-triangle heightfield at 640x480, 1 spp (1.16 G nodes): 254 ->
 // 65 ms, at 160x120 (72 M): 22.6 -> 4.6; a 64x64-vertex heightfield at
 // 128x96, 8 spp (53 M): 7.9 -> 5.4; a room of smooth spheres (28 M nodes, 90
-// per point): 6.0 -> 5.3.  24 of 32 lanes are active (10 before).  Without
+// per point): 6.0 -> 5.3.  22.3 of 32 lanes are active (10 before).  Without
 // the rounds the first took 184 ms and the second 20.7 (its few longest walks
 // ran alone); with one step for every node that splits or draws 83 and 5.9.
 #pragma once

@@ -395,8 +395,9 @@ DEV BounceHit sample_bsdf_scene(const DevScene &s, const BSDFSample &bs, float3 
 // Step says how a path starts a bounce: on its own, or with the paths of its
 // block (every thread calls then, those without a path with alive = false), so
 // that the block's warps fetch the bounce's instructions together.  A path on
-// its own leaves the loop where it ends (soft shadow image, 640x480x8 samples:
-// 0.764 ms, 0.773 with the flag tested at the next bounce).
+// its own leaves the loop where it ends and a sample where it misses (mirror
+// hall, 512x384x4 samples, five bounces: 0.962 ms, 0.970 where a miss runs on to
+// the loop's test; soft shadow, 640x480x8, three bounces: 0.664 and 0.676).
 struct OwnStep {
     static constexpr bool kOwn = true;
     DEV static bool any(bool) { return true; }
